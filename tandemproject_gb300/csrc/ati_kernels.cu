@@ -18,6 +18,7 @@
 #include <utility>
 
 #include "ati_convert.h"
+#include "ati_fixed.h"
 #include "ati_kernels.h"
 #include "ati_tma.h"
 
@@ -3001,9 +3002,17 @@ __global__ void k_metric_div(const double *d3, int64_t N, float *gm) {
 template <typename TI, typename TO, typename TC>
 static void sweep_t(const Eng<TC> &e, cudaStream_t st, int nn, bool filt, const SweepIO<TI, TO> &io) {
   if (e.nlt[nn] == 0) return;
+  int first = 0;  // first tile of the sequential kernels
+  if constexpr (kFast && std::is_same<TC, double>::value) {
+    if (e.fx_ok[filt][nn]) {
+      fast::sweep_fixed(e, st, nn, filt, io);
+      if (e.nlt[nn] == e.nlt_fx[nn]) return;
+      first = e.nlt_fx[nn];  // lines too short or long for them
+    }
+  }
   SweepArgs<TI, TO, TC> a;
   a.blk = e.blk;
-  a.lt = e.lt[nn];
+  a.lt = e.lt[nn] + first;
   a.cf = e.cf;
   a.fac = filt ? e.facf : e.facd;
   a.facu = filt ? e.facuf : e.facud;
@@ -3084,7 +3093,7 @@ static void sweep_t(const Eng<TC> &e, cudaStream_t st, int nn, bool filt, const 
       return;
     }
   }
-  const dim3 grid(e.nlt[nn], io.nf);
+  const dim3 grid(e.nlt[nn] - first, io.nf);
   if (nn == 1) {
     if (filt) k_sweep_xc<true, TI, TO, TC><<<grid, XC_NL, 0, st>>>(a);
     else k_sweep_xc<false, TI, TO, TC><<<grid, XC_NL, 0, st>>>(a);

@@ -34,6 +34,7 @@ constexpr int PW_KINDS = 7;
 // The segmented sweeps' tiles of one direction fall into classes of blocks whose lines have the same segment
 // count (a batch mixes line lengths): one launch per class, with the warps and shared memory of the class's
 // longest line.  A class is tiles [off, off + n) of lts, lines of up to maxlen points, groups line groups a CTA.
+// (FP64 handles, whose fixed-point sweeps take the same tiles, have one group a CTA.)
 struct SegClass {
   int off, n, maxlen, groups;
 };
@@ -58,6 +59,12 @@ struct Eng {
   int dzl;                   // their largest line length (0: the dense zeta sweep is not available)
   bool dense;                // the zeta derivative sweeps take the dense operators (ATI_OPT_DENSE_ZETA)
   const double *facud, *facuf;  // FP64 fast path: scaled-factor row tables (FU_RT per row; derivative, filter)
+  // FP64 fast path: fixed-point line sweeps (ati_fixed.h) for [derivative, filter] of each direction, their tables
+  bool fx_ok[2][4];
+  int nlt_fx[4];        // leading tiles of lt[nn] whose blocks those sweeps take (the others' lines are too short or long)
+  const int *fxr[2];
+  const int64_t *fxe[2];
+  int fx_gbits[2], fx_k[2];
   int sg_lines[4];      // lines per CTA of the eta (2) and zeta (3) sweeps: the tiles of lt[2], lt[3]
   int maxlen[4];        // longest line per direction
   int64_t N;            // points of all blocks
