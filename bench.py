@@ -65,15 +65,15 @@ FIELD_SWEEPS_PER_STEP = {"deriv": 4 * (4 + 5), "filter": 5}
 # 3.54 M-point case: 489.35 MB for 17.69 M units); the kernel streams, so the
 # traffic of a launch scales with the units it processes
 SWEEP_TRAFFIC_PER_UNIT = {"deriv_xi": 489.35e6 / (5 * 3538944)}
-# DRAM bytes per point of k_flux_visc measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum of one launch
+# DRAM bytes per point of the viscous flux kernel (k_flux_fixed) measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum of one launch
 # on the 3.54 M-point case: 906.4 + 395.5 MB); the kernel streams, so the traffic scales with the points
 FLUX_TRAFFIC_PER_POINT = (906.36e6 + 395.46e6) / 3538944
-# algorithmic bytes per point of the FP64 fast path's viscous flux kernel k_flux_visc (the stresses of k_visc taken
+# algorithmic bytes per point of the FP64 fast path's viscous flux kernel k_flux_fixed (the stresses of k_visc taken
 # at the point): it reads the metrics (72 B), the twelve derivative planes of u, v, w, T (96 B), Jacobian and
 # viscosity (16 B), velocity (24 B), pressure (8 B) and the state (40 B), and writes 15 fluxes (120 B)
 FLUX_BYTES_FP64 = 376
-# its FP64 flops per point (an FMA counts two), from ncu's opcode counts of one launch on the 3.54 M-point case:
-# 81 DFMA, 42 DMUL and 15 DADD a point
+# the FP64 flops per point (an FMA counts two) of the same fluxes in FP64 arithmetic, 81 DFMA, 42 DMUL and 15 DADD a
+# point; the kernel does them in 64-bit fixed point
 FLUX_FLOPS_FP64 = 219
 # canonical bytes per grid-point-stage of the whole stage: 141 FP64 words, or
 # the mixed data flow with FP32 intermediates and FP64 state/metrics
@@ -512,7 +512,7 @@ def main():
 
     sweep_cls = max((k for k in prof if k.startswith(("deriv", "filter")) and prof[k][1]), key=lambda k: prof[k][0])
     if dom == "flux" and cfg.nviscous == 1:
-        # the viscous flux kernel with the stresses at the point (k_flux_visc): one launch covers every point
+        # the viscous flux kernel with the stresses at the point (k_flux_fixed): one launch covers every point
         ms, n = prof["flux"]
         t = ms / max(n, 1) / 1e3
         achieved = FLUX_BYTES_FP64 * npts / t / 1e9
@@ -522,7 +522,7 @@ def main():
                     "traffic": FLUX_TRAFFIC_PER_POINT * npts if FLUX_TRAFFIC_PER_POINT else None,
                     "traffic_source": "ncu DRAM bytes per point of one launch on the 3.54 M-point case, scaled by "
                                       "points",
-                    "kernel": f"k_flux_visc (viscous fluxes with the stresses at the point): one launch = every point "
+                    "kernel": f"k_flux_fixed (viscous fluxes with the stresses at the point): one launch = every point "
                               f"({npts}), {FLUX_BYTES_FP64} B and {FLUX_FLOPS_FP64} FP64 flop per point",
                     "fp64": {"achieved_tflops": fp64_ach, "peak_tflops": fp64_peak, "frac": fp64_ach / fp64_peak}}
     elif dom.startswith(("deriv", "filter")):
@@ -533,8 +533,8 @@ def main():
     roofline["fp64"]["peak_source"] = "measured FP64 FMA throughput of this GPU (ati_probe_fma_tflops)"
     roofline.update({
         "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)",
-        "limit": "the FP64 pipe (ncu: 89-92 % busy in the line sweeps and the flux kernel at 12-34 % of HBM); "
-                 "frac is against HBM, fp64.frac against the FP64 FMA peak",
+        "limit": "integer issue: the line sweeps and the fluxes run in 64-bit fixed point on the integer pipes; frac is "
+                 "against HBM, fp64 the rate of the same work counted in FP64 operations against the FP64 FMA peak",
         "stage_hbm_frac": STAGE_BYTES_FP64 * value / ws / 1e9 / hbm_peak,
         "kernel_share": {k: round(v[0] / tot, 4) for k, v in prof.items() if v[1]}})
     if dom != sweep_cls and "note" not in roofline:

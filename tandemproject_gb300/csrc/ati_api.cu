@@ -1360,6 +1360,7 @@ static int create_impl(const ati_config_t *cfgs, int ncase, ati_handle_t **out) 
     for (int c = 0; c < SEG_NCLASS; c++) d.segc[nn][c] = h->segc[nn][c];
   }
   d.eta_rowtiles = h->tma[2];
+  d.fx_flux = h->cfg.precision != ATI_FP64 || h->cfg.les == 1 ? 0 : (h->cfg.nviscous == 1 ? 1 : 2);
   for (int q = 0; q < 2; q++) {
     for (int nn = 1; nn <= 3; nn++) d.fx_ok[q][nn] = fix[q].ok[nn];
     d.fxr[q] = (const int *)(h->arena + o_fxr[q]) + FX_PAD * FX_RT;

@@ -19,6 +19,7 @@
 
 #include "ati_convert.h"
 #include "ati_fixed.h"
+#include "ati_fixed_flux.h"
 #include "ati_kernels.h"
 #include "ati_tma.h"
 
@@ -2088,7 +2089,8 @@ __device__ __forceinline__ void flux_fast_point(const Eng<double> &e, int64_t N,
 // (src/Main3D.f90:710-766): flx plane (m-1)*3 + (nn-1)
 // (the FP32 kernel streams: five CTAs of 256 threads an SM, at most 51 registers a thread, keep more loads
 // in flight than the 80 registers it would take unbounded; measured 380 -> 296 us a launch on 8.85 M points)
-// (the mixed path's viscous fluxes take the stresses at the point instead: k_flux_staged)
+// (the mixed path's viscous fluxes take the stresses at the point instead: k_flux_staged; the FP64 fast path's run in fixed
+// point, k_flux_fixed, but with the LES terms)
 template <typename R>
 __global__ void __launch_bounds__(256, Freestream<R>::on ? 5 : 1) k_flux(Eng<R> e) {
   const int64_t N = e.N;
@@ -2179,19 +2181,52 @@ __global__ void __launch_bounds__(256, Freestream<R>::on ? 5 : 1) k_flux(Eng<R> 
   }
 }
 
-// the FP64 fast path's viscous fluxes with the stresses taken at the point (k_visc and k_flux in one pass: the
-// nine stress planes are neither written nor read)
-__global__ void __launch_bounds__(256) k_flux_visc(Eng<double> e) {
+// the FP64 fast path's fluxes in fixed point (flux_point_fixed), the viscous ones with the stresses at the point (no
+// stress plane is written or read); points whose values leave its range take the FP64 operations.  On 8.85 M points
+// 2131 -> 830 us a launch against the FP64 kernel, whose 138 operations a point kept the FP64 pipe 91 % busy; 376 B a
+// point, 4.0 TB/s.  Two CTAs of 256 threads an SM, 128 registers: one CTA (255 registers) 959 us, three (85) 1060 us.
+template <bool VISC>
+__device__ __noinline__ void flux_point_fp64(const Eng<double> &e, int64_t g, double u1, double u2, double u3,
+                                             const ViscConst<double> &V) {
+  flux_fast_point<VISC, VISC>(e, e.N, g, u1, u2, u3, &V);
+}
+template <bool VISC>
+__global__ void __launch_bounds__(256, 2) k_flux_fixed(const __grid_constant__ Eng<double> e) {
   const int64_t N = e.N;
   TILE_LOOP(e, T) {
     const Scheme &S = e.sc[T.cs];
     const Scalars &SC = e.scal[T.cs];
-    const double u1 = SC.umf[1], u2 = SC.umf[2], u3 = SC.umf[3];
-    if (S.nviscous == 1) {
-      const ViscConst<double> V(S);
-      POINT_LOOP(T, g) flux_fast_point<true, true>(e, N, g, u1, u2, u3, &V);
-    } else {
-      POINT_LOOP(T, g) flux_fast_point<false>(e, N, g, u1, u2, u3);
+    FluxIn I;
+    I.umf[0] = SC.umf[1];
+    I.umf[1] = SC.umf[2];
+    I.umf[2] = SC.umf[3];
+    const ViscConst<double> V(S);
+    POINT_LOOP(T, g) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        I.m[0][k] = e.xim[g + k * N];
+        I.m[1][k] = e.etm[g + k * N];
+        I.m[2][k] = e.zem[g + k * N];
+        I.vel[k] = e.prim[g + k * N];
+      }
+      if (VISC) {
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+#pragma unroll
+          for (int n = 0; n < 3; n++) I.dv[f][n] = e.dv[g + (f * 3 + n) * N];
+        I.r1 = e.mu[g] * e.yaco[g];
+        I.r2 = V.gp * I.r1;
+      }
+      I.p = e.p[g];
+#pragma unroll
+      for (int k = 0; k < 5; k++) I.q[k] = e.qa[g + k * N];
+      double F[15];
+      if (flux_point_fixed<VISC>(I, F)) {
+#pragma unroll
+        for (int c = 0; c < 15; c++) e.flx[g + c * N] = F[c];
+      } else {
+        flux_point_fp64<VISC>(e, g, I.umf[0], I.umf[1], I.umf[2], V);
+      }
     }
   }
 }
@@ -3212,10 +3247,18 @@ static void pointwise_t(const Eng<R> &eng, cudaStream_t st, int which) {
       break;
     case PW_CFL: k_cfl<R><<<g, t, 0, st>>>(e); break;
     case PW_VISC: k_visc<R><<<g, t, 0, st>>>(e); break;
-    case PW_FLUX: k_flux<R><<<g, t, 0, st>>>(e); break;
-    case PW_FLUX_STRESS:  // viscous fluxes with the stresses taken at the point (the strict FP64 path: k_visc)
+    case PW_FLUX:
+    case PW_FLUX_STRESS:
+      if constexpr (kFast && !Freestream<R>::on) {  // (the stresses at the point, whether or not k_visc wrote its planes)
+        if (e.fx_flux == 1) k_flux_fixed<true><<<g, t, 0, st>>>(e);
+        else if (e.fx_flux == 2) k_flux_fixed<false><<<g, t, 0, st>>>(e);
+        if (e.fx_flux) break;
+      }
+      if (which == PW_FLUX) {
+        k_flux<R><<<g, t, 0, st>>>(e);
+        break;
+      }
       if constexpr (Freestream<R>::on) k_flux_staged<<<g, t, flux_staged_smem(t), st>>>(e);
-      else if constexpr (kFast) k_flux_visc<<<g, t, 0, st>>>(e);
       break;
     case PW_DIV: k_div<R><<<g, t, 0, st>>>(e); break;
     case PW_RK: k_rk<R><<<g, t, 0, st>>>(e); break;

@@ -65,6 +65,7 @@ struct Eng {
   const int *fxr[2];
   const int64_t *fxe[2];
   int fx_gbits[2], fx_k[2];
+  int fx_flux;          // its fluxes: 1 viscous, 2 inviscid in fixed point (ati_fixed_flux.h), 0 FP64 (LES; strict mode)
   int sg_lines[4];      // lines per CTA of the eta (2) and zeta (3) sweeps: the tiles of lt[2], lt[3]
   int maxlen[4];        // longest line per direction
   int64_t N;            // points of all blocks

@@ -1,9 +1,10 @@
-"""The fixed-point line sweeps of the FP64 fast path (csrc/ati_fixed.cu) against the CPU restatement.
+"""The fixed-point line sweeps (csrc/ati_fixed.cu) and fluxes (csrc/ati_fixed_flux.h) of the FP64 fast path against the
+CPU restatement.
 
 Line lengths sit at the edges of the kernel's segments (48 points a segment, tiles of 32 lines, lines of 13 to 800
 points; others take the FP64 sweeps).  The tolerances are those of the FP64 fast build: a filter step adds a
 correction rounded well below an ulp of the state (1e-14 of each variable's norm), a stage's right-hand side nearly
-cancels, so the state after two steps is held to 1e-12.
+cancels, so the state after two steps is held to 1e-12 and a stage's right-hand side to 1e-9 of its largest value.
 """
 import numpy as np
 import pytest
@@ -114,4 +115,28 @@ def test_filter_spreads_a_nan_as_the_oracle_does(ati_lib, oracle_lib):
         assert np.array_equal(np.isfinite(a), np.isfinite(b))
         ok = np.isfinite(b)
         assert rel_err(a[ok], b[ok]) < 1e-14
+    gpu.close()
+
+
+@pytest.mark.parametrize("viscous", [1, 0])
+@pytest.mark.parametrize("pressure,speed", [(1.0, 1.0), (1.0, 0.0), (1e-40, 1e-20), (1e66, 1e33)])
+def test_right_hand_side_matches_oracle(ati_lib, oracle_lib, viscous, pressure, speed):
+    """One stage (dt = 0 before the first step: the state stays) of flows at all scales: within the fixed-point
+    fluxes' exponent range, at rest, near its lower end, and beyond the upper one (the FP64 operations)."""
+    from tandemproject_gb300.solver import F_DE
+    cfg = small_case(lxibk=(30, 70, 24), letbk=(17, 20), lzebk=(12,), nviscous=viscous)
+    gpu, orc, g = pair(cfg)
+    for mb in range(cfg.nblocks):
+        q = smooth_state(g[mb], 11)
+        kinetic = 0.5 * (q[1] ** 2 + q[2] ** 2 + q[3] ** 2) / q[0]
+        q[4] = (q[4] - kinetic) * pressure + kinetic * speed ** 2
+        q[1:4] *= speed
+        gpu.set_state(mb, q)
+        orc.set_state(mb, q)
+    gpu.rk_stage(1)
+    orc.rk_stage(1)
+    for mb in range(cfg.nblocks):
+        a, b = gpu.get_field(mb, F_DE), orc.get_field(mb, F_DE).reshape(5, -1)
+        for m in range(5):
+            assert rel_err(a[m], b[m]) < 1e-9, (mb, m)
     gpu.close()
