@@ -140,3 +140,42 @@ def test_right_hand_side_matches_oracle(ati_lib, oracle_lib, viscous, pressure, 
         for m in range(5):
             assert rel_err(a[m], b[m]) < 1e-9, (mb, m)
     gpu.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-9, 1e25, 1e70])
+def test_pressure_matches_oracle_pointwise(ati_lib, oracle_lib, scale):
+    """The fixed-point primitives, and the FP64 ones beyond their range (1e70), point by point: p is (gamma - 1) times
+    the energy less the kinetic one, 2 to 5 units in the last place with the cancellation of these states."""
+    from tandemproject_gb300.solver import F_P
+    cfg = small_case(lxibk=(30, 70, 24), letbk=(17, 20), lzebk=(12,))
+    gpu, orc, g = pair(cfg)
+    for mb in range(cfg.nblocks):
+        q = smooth_state(g[mb], 2)
+        q[1:4] *= scale ** 0.5
+        q[4] *= scale
+        gpu.set_state(mb, q)
+        orc.set_state(mb, q)
+    gpu.rk_stage(1)
+    orc.rk_stage(1)
+    for mb in range(cfg.nblocks):
+        a, b = gpu.get_field(mb, F_P), orc.get_field(mb, F_P).reshape(1, -1)
+        assert np.max(np.abs(a / b - 1)) < 1e-14, mb
+    gpu.close()
+
+
+def test_negative_pressure_is_flagged(ati_lib):
+    from tandemproject_gb300.solver import ATI_ENONFINITE, AtiError, Case
+    cfg = small_case(lxibk=(30, 70, 24), letbk=(17, 20), lzebk=(12,))
+    g = aerofoil_grid(cfg)
+    gpu = Case(cfg)
+    for mb in range(cfg.nblocks):
+        gpu.set_grid(mb, g[mb])
+    gpu.init()
+    q = smooth_state(g[2], 2)
+    q[4, 777] = 0.5 * (q[1, 777] ** 2) / q[0, 777] * 0.5
+    gpu.set_state(2, q)
+    gpu.rk_stage(1)
+    with pytest.raises(AtiError) as err:
+        gpu.check()
+    assert err.value.code == ATI_ENONFINITE
+    gpu.close()
