@@ -402,15 +402,15 @@ int ati_check_recip(int64_t n, double worst[2]);
  * codes 35, 40 or 45 (ndf = 1) take closure rows instead and differ --
  * asynchronously on `stream` (a cudaStream_t; NULL = the legacy default
  * stream).
- *  - Allocates and frees nothing.  Its scratch (LU factors and the
- *    forward-elimination values) is one static device array of
- *    5*ATI_NOALLOC_MAX_LEN + ATI_NOALLOC_MAX_POINTS doubles (about 16 MB)
- *    per GPU, held until the process exits.
+ *  - Allocates and frees nothing.  Its scratch (LU factors; the
+ *    forward-elimination values stay in shared memory) is one static device
+ *    array of 5*ATI_NOALLOC_MAX_LEN doubles (160 KB) per GPU, held until the
+ *    process exits.
  *  - The first call on each device (and again after a device reset, which
  *    gives the context a new array) looks up the array's device address with
  *    cudaGetSymbolAddress, that device current.  Under CUDA's default lazy
  *    module loading that look-up is also when the driver loads the module and
- *    reserves the 16 MB, so the first call can fail with ATI_ECUDA on a device
+ *    reserves the array, so the first call can fail with ATI_ECUDA on a device
  *    with no room left: make one call (nlines may be 1) before a memory pool
  *    takes the device's memory and before any stream capture, or set
  *    CUDA_MODULE_LOADING=EAGER so that the array is reserved when the context

@@ -6,15 +6,15 @@
 // (a device allocation can synchronise the whole device and can fail late,
 // when memory is fragmented).  ati_deriv_lines_noalloc serves them: the
 // caller passes its own input and output arrays, and the only extra memory
-// the kernel needs -- the LU factor table and the forward-elimination values
-// -- lives in the file-scope device array below (about 16 MB on every GPU that
-// uses it, held until the process exits).  No call allocates or frees anything.
+// the kernel needs -- the LU factor table -- lives in the file-scope device
+// array below (160 KB on every GPU that uses it, held until the process exits);
+// the forward-elimination values stay in shared memory.  No call allocates or frees anything.
 //
 // When the array is reserved: with CUDA's default lazy module loading this file's
 // module, and the array with it, is loaded into a context the first time the
 // module is used there, which is the first call's address look-up.  That first
-// call on a device therefore reserves the 16 MB, and it fails with ATI_ECUDA if
-// the device has no 16 MB left.  A caller whose own pool takes the device memory
+// call on a device therefore reserves the array, and it fails with ATI_ECUDA if
+// the device has no room left.  A caller whose own pool takes the device memory
 // makes one call (nlines may be 1) before the pool does, and before any stream
 // capture; with CUDA_MODULE_LOADING=EAGER in the environment the driver reserves
 // the array when the context is created instead.
@@ -36,9 +36,9 @@ namespace {
 
 constexpr int64_t kMaxPoints = ATI_NOALLOC_MAX_POINTS;
 constexpr int kMaxLen = ATI_NOALLOC_MAX_LEN;
-constexpr int64_t kScratchDoubles = 5 * (int64_t)kMaxLen + kMaxPoints;
+constexpr int64_t kScratchDoubles = 5 * (int64_t)kMaxLen;
 
-// factor table (5 per line position) followed by the forward-elimination plane
+// factor table (5 per line position)
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
 constexpr double kAlpha = 0.5862704032801503, kBeta = 0.09549533555017055;
@@ -94,69 +94,98 @@ __global__ void k_noalloc_factors(double *fac, int len, Rows R) {
   }
 }
 
-// one thread per contiguous line: RHS, forward elimination into the scratch
-// plane, back substitution into the caller's output
-__global__ void k_noalloc_deriv(const double *in, double *out, int64_t nlines, int len, const double *fac,
-                                double *fw, Rows R) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nlines) return;
-  const int L = len;
-  const double *p = in + t * L;
-  double *w = fw + t * L;
-  double *o = out + t * L;
-  const double *a;
-  double sbs0, sbs1, sbs2, sbe0, sbe1, sbe2;
-  {
-    const double w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4], w5 = p[5], w6 = p[6];
-    a = R.abc[0];
-    sbs0 = a[0] * (w1 - w0) + a[1] * (w2 - w0) + a[2] * (w3 - w0) + a[3] * (w4 - w0) + a[4] * (w5 - w0) + a[5] * (w6 - w0);
-    a = R.abc[1];
-    sbs1 = a[0] * (w0 - w1) + a[1] * (w2 - w1) + a[2] * (w3 - w1) + a[3] * (w4 - w1) + a[4] * (w5 - w1) + a[5] * (w6 - w1);
-    a = R.abc[2];
-    sbs2 = a[0] * (w0 - w2) + a[1] * (w1 - w2) + a[2] * (w3 - w2) + a[3] * (w4 - w2) + a[4] * (w5 - w2) + a[5] * (w6 - w2);
+// A CTA takes LPC contiguous lines.  The right-hand sides, independent of one another, are formed by all threads from
+// coalesced loads into a shared-memory tile (one line a row, odd pitch); the recurrences, serial along a line, run in
+// one warp, lane l line l, on the tile; the back substitution's products c2 w are again formed by all threads, and the
+// results leave coalesced.  Bound: a warp FP64 operation takes 64 clocks whatever its active lanes, and a row's
+// recurrences are four of them each way, in the order of deriv (the results equal ati_deriv's bit for bit).
+// Few lines a CTA spread the recurrence warps over the SMs' four sub-partitions: the warp that runs them is the
+// CTA's rank on its SM modulo four (CTAs b and b + nsm share an SM).  Measured, 3327 lines of 601 points: 726 us with
+// one thread a line on global memory (uncoalesced), now 251; 40 lines of 97: 65 us, now 43.
+constexpr int kThreads = 128;
+__global__ void __launch_bounds__(kThreads) k_noalloc_deriv(const double *in, double *out, int64_t nlines, int len,
+                                                            int lpc, int nsm, const double *fac, Rows R) {
+  extern __shared__ double tile[];
+  const int L = len, P = len | 1, t = (int)threadIdx.x;
+  const int64_t l0 = (int64_t)blockIdx.x * lpc;
+  const int n = (int)(nlines - l0 < lpc ? nlines - l0 : lpc);
+  const double *p0 = in + l0 * L;
+  for (int ln = 0; ln < n; ln++) {
+    const double *p = p0 + (int64_t)ln * L;
+    double *o = tile + ln * P;
+    for (int i = t + 3; i <= L - 4; i += kThreads)
+      o[i] = kAa * (p[i + 1] - p[i - 1]) + kAb * (p[i + 2] - p[i - 2]) + kAc * (p[i + 3] - p[i - 3]);
   }
-  {
-    const double w0 = p[L - 1], w1 = p[L - 2], w2 = p[L - 3], w3 = p[L - 4], w4 = p[L - 5], w5 = p[L - 6], w6 = p[L - 7];
-    a = R.abc[0];
-    sbe0 = a[0] * (w0 - w1) + a[1] * (w0 - w2) + a[2] * (w0 - w3) + a[3] * (w0 - w4) + a[4] * (w0 - w5) + a[5] * (w0 - w6);
-    a = R.abc[1];
-    sbe1 = a[0] * (w1 - w0) + a[1] * (w1 - w2) + a[2] * (w1 - w3) + a[3] * (w1 - w4) + a[4] * (w1 - w5) + a[5] * (w1 - w6);
-    a = R.abc[2];
-    sbe2 = a[0] * (w2 - w0) + a[1] * (w2 - w1) + a[2] * (w2 - w3) + a[3] * (w2 - w4) + a[4] * (w2 - w5) + a[5] * (w2 - w6);
+  for (int q = t; q < 2 * n; q += kThreads) {  // closure rows, one line end a thread
+    const int ln = q >> 1, end = q & 1;
+    const double *p = p0 + (int64_t)ln * L;
+    double *o = tile + ln * P;
+    const double *a;
+    double s0, s1, s2;
+    if (!end) {
+      const double w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4], w5 = p[5], w6 = p[6];
+      a = R.abc[0];
+      s0 = a[0] * (w1 - w0) + a[1] * (w2 - w0) + a[2] * (w3 - w0) + a[3] * (w4 - w0) + a[4] * (w5 - w0) + a[5] * (w6 - w0);
+      a = R.abc[1];
+      s1 = a[0] * (w0 - w1) + a[1] * (w2 - w1) + a[2] * (w3 - w1) + a[3] * (w4 - w1) + a[4] * (w5 - w1) + a[5] * (w6 - w1);
+      a = R.abc[2];
+      s2 = a[0] * (w0 - w2) + a[1] * (w1 - w2) + a[2] * (w3 - w2) + a[3] * (w4 - w2) + a[4] * (w5 - w2) + a[5] * (w6 - w2);
+      o[0] = s0; o[1] = s1; o[2] = s2;
+    } else {
+      const double w0 = p[L - 1], w1 = p[L - 2], w2 = p[L - 3], w3 = p[L - 4], w4 = p[L - 5], w5 = p[L - 6], w6 = p[L - 7];
+      a = R.abc[0];
+      s0 = a[0] * (w0 - w1) + a[1] * (w0 - w2) + a[2] * (w0 - w3) + a[3] * (w0 - w4) + a[4] * (w0 - w5) + a[5] * (w0 - w6);
+      a = R.abc[1];
+      s1 = a[0] * (w1 - w0) + a[1] * (w1 - w2) + a[2] * (w1 - w3) + a[3] * (w1 - w4) + a[4] * (w1 - w5) + a[5] * (w1 - w6);
+      a = R.abc[2];
+      s2 = a[0] * (w2 - w0) + a[1] * (w2 - w1) + a[2] * (w2 - w3) + a[3] * (w2 - w4) + a[4] * (w2 - w5) + a[5] * (w2 - w6);
+      o[L - 1] = s0; o[L - 2] = s1; o[L - 3] = s2;
+    }
   }
-  double f2 = sbs0, f1 = sbs1 - fac[1 * 5 + 1] * f2;
-  w[0] = f2;
-  w[1] = f1;
-  {
-    const double v = sbs2 - fac[2 * 5 + 0] * f2 - fac[2 * 5 + 1] * f1;
-    w[2] = v;
-    f2 = f1; f1 = v;
+  __syncthreads();
+  const int lane = t & 31;
+  const bool serial = (t >> 5) == (int)((blockIdx.x / nsm) & 3u) && lane < n;
+  double *w = tile + (serial ? lane : 0) * P;
+  if (serial) {
+    double f2 = w[0], f1 = w[1] - __ldg(fac + 6) * f2;
+    w[1] = f1;
+#pragma unroll 4
+    for (int i = 2; i < L; i++) {
+      const double v = w[i] - __ldg(fac + i * 5) * f2 - __ldg(fac + i * 5 + 1) * f1;
+      w[i] = v;
+      f2 = f1;
+      f1 = v;
+    }
   }
-  double a0 = p[0], a1 = p[1], a2 = p[2], a3 = p[3], a4 = p[4], a5 = p[5];
-  for (int i = 3; i <= L - 4; i++) {
-    const double a6 = p[i + 3];
-    const double sb = kAa * (a4 - a2) + kAb * (a5 - a1) + kAc * (a6 - a0);
-    const double v = sb - fac[i * 5 + 0] * f2 - fac[i * 5 + 1] * f1;
-    w[i] = v;
-    f2 = f1; f1 = v;
-    a0 = a1; a1 = a2; a2 = a3; a3 = a4; a4 = a5; a5 = a6;
+  __syncthreads();
+  for (int ln = 0; ln < n; ln++)
+    for (int i = t; i < L; i += kThreads) tile[ln * P + i] = __ldg(fac + i * 5 + 2) * tile[ln * P + i];
+  __syncthreads();
+  if (serial) {
+    double b0 = w[L - 1], b1 = w[L - 2] - __ldg(fac + (L - 2) * 5 + 3) * b0;
+    w[L - 2] = b1;
+#pragma unroll 4
+    for (int i = L - 3; i >= 0; i--) {
+      const double v = w[i] - __ldg(fac + i * 5 + 3) * b1 - __ldg(fac + i * 5 + 4) * b0;
+      w[i] = v;
+      b0 = b1;
+      b1 = v;
+    }
   }
-  const double sbe[3] = {sbe2, sbe1, sbe0};
-  for (int r = 0; r < 3; r++) {
-    const int i = L - 3 + r;
-    const double v = sbe[r] - fac[i * 5 + 0] * f2 - fac[i * 5 + 1] * f1;
-    if (r < 2) w[i] = v;
-    f2 = f1; f1 = v;
-  }
-  double b0 = fac[(L - 1) * 5 + 2] * f1;
-  double b1 = fac[(L - 2) * 5 + 2] * f2 - fac[(L - 2) * 5 + 3] * b0;
-  o[L - 1] = b0;
-  o[L - 2] = b1;
-  for (int i = L - 3; i >= 0; i--) {
-    const double v = fac[i * 5 + 2] * w[i] - fac[i * 5 + 3] * b1 - fac[i * 5 + 4] * b0;
-    o[i] = v;
-    b0 = b1; b1 = v;
-  }
+  __syncthreads();
+  double *q0 = out + l0 * L;
+  for (int ln = 0; ln < n; ln++)
+    for (int i = t; i < L; i += kThreads) q0[(int64_t)ln * L + i] = tile[ln * P + i];
+}
+
+// lines a CTA: the fewest (4 to 32) that leave at most one recurrence warp a sub-partition of the device, within the
+// shared memory of a CTA
+constexpr size_t kTileMax = 200 * 1024;
+int lines_per_cta(int64_t nlines, int len, int nsm) {
+  int lpc = 4;
+  while (lpc < 32 && (nlines + lpc - 1) / lpc > 4 * (int64_t)nsm) lpc *= 2;
+  while (lpc > 4 && (size_t)lpc * (len | 1) * sizeof(double) > kTileMax) lpc /= 2;
+  return lpc;
 }
 
 std::mutex g_mu;
@@ -165,6 +194,7 @@ std::mutex g_mu;
 void *g_ptr[64] = {nullptr};
 void *g_ctx[64] = {nullptr};
 int g_len[64];
+int g_nsm[64];
 bool g_len_init = false;
 
 // cuCtxGetCurrent from the driver, fetched through the runtime (no link-time dependency on libcuda): a device
@@ -239,6 +269,7 @@ extern "C" int ati_deriv_lines_noalloc(const double *in, double *out, int64_t nl
   }
   void *base = nullptr;
   bool refactor = false;
+  int nsm = 1;
   {
     // set-up, once per device and context: look up the device address of the scratch array with that device
     // current (in host code the symbol itself is only a host-side stand-in, not a device address)
@@ -256,23 +287,34 @@ extern "C" int ati_deriv_lines_noalloc(const double *in, double *out, int64_t nl
                                           "failed: ") + cudaGetErrorString(e)).c_str());
         return ATI_ECUDA;
       }
+      // (a context's kernels have their own attributes: set with the look-up)
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_noalloc_deriv, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)kTileMax);
+      int nsm = 0;
+      if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+      if (e != cudaSuccess) {
+        ati_set_thread_error((std::string("ati_deriv_lines_noalloc: ") + cudaGetErrorString(e)).c_str());
+        return ATI_ECUDA;
+      }
+      g_nsm[dev] = nsm > 0 ? nsm : 1;
       if (p != g_ptr[dev]) g_len[dev] = -1;  // a new array: no factors yet
       g_ptr[dev] = p;
       g_ctx[dev] = current_ctx();
     }
     base = g_ptr[dev];
+    nsm = g_nsm[dev];
     refactor = g_len[dev] != len;
     g_len[dev] = len;
   }
   double *fac = (double *)base;
-  double *fw = fac + 5 * (int64_t)kMaxLen;
   cudaStream_t st = (cudaStream_t)stream;
   const Rows R = make_rows();
   // the LU factors depend on the line length only: refactored when it changes (calls are ordered on the GPU, so
   // a call finds the factors of the previous call in the array)
   if (refactor) k_noalloc_factors<<<1, 1, 0, st>>>(fac, len, R);
-  const int tpb = 128;
-  k_noalloc_deriv<<<(unsigned)((nlines + tpb - 1) / tpb), tpb, 0, st>>>(in, out, nlines, len, fac, fw, R);
+  const int lpc = lines_per_cta(nlines, len, nsm);
+  const size_t smem = (size_t)lpc * (len | 1) * sizeof(double);
+  k_noalloc_deriv<<<(unsigned)((nlines + lpc - 1) / lpc), kThreads, smem, st>>>(in, out, nlines, len, lpc, nsm, fac, R);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     std::lock_guard<std::mutex> lk(g_mu);
