@@ -1401,7 +1401,7 @@ static int create_impl(const ati_config_t *cfgs, int ncase, ati_handle_t **out) 
     m.dense = false;
     m.tmaps = (const TmaMap *)(h->arena + o_tmap);
     m.nblk = h->nb;
-    for (int nn = 0; nn < 4; nn++) m.tma[nn] = h->tma[nn];
+    m.tma[2] = h->tma[2];  // (zeta tiles come in faster by the threads' own copies: only where the caller asks for TMA)
     m.eta_rowtiles = h->tma[2];
     m.pairs = true;
   }

@@ -33,6 +33,9 @@ __global__ void k_check_conv(int64_t n, unsigned long long *bad) {
     const float f = __uint_as_float(fb);
     const double wa = ati::widen(f), wb = (double)f;
     if (!((wa != wa && wb != wb) || __double_as_longlong(wa) == __double_as_longlong(wb))) nb++;
+    double wv[1];
+    ati::widen_all<1>({f}, wv);
+    if (!((wv[0] != wv[0] && wb != wb) || __double_as_longlong(wv[0]) == __double_as_longlong(wb))) nb++;
     // narrowing: random doubles over the whole exponent range, exact ties and near-ties of the dropped 29 bits,
     // the edges of the normal float range, zeros, infinities and NaNs
     const uint64_t r2 = mix64(r ^ 0xD1B54A32D192ED03ull);
@@ -50,6 +53,9 @@ __global__ void k_check_conv(int64_t n, unsigned long long *bad) {
     const double d = __longlong_as_double((long long)db);
     const float na = ati::narrow(d), nb2 = (float)d;
     if (!((na != na && nb2 != nb2) || __float_as_uint(na) == __float_as_uint(nb2))) nb++;
+    float nv[1];
+    ati::narrow_all<1>({d}, nv);
+    if (!((nv[0] != nv[0] && nb2 != nb2) || __float_as_uint(nv[0]) == __float_as_uint(nb2))) nb++;
   }
   if (nb) atomicAdd(bad, nb);
 }

@@ -69,6 +69,47 @@ __device__ __forceinline__ double rsqrt_nr(double a) {
   return y;
 }
 
+// (an instruction the compiler cannot predicate: the block that holds it stays behind a branch)
+__device__ __forceinline__ void keep_branch() { asm volatile("nanosleep.u32 0;"); }
+
+// K conversions at a time, the values outside the integer forms' range behind one branch (zeros, subnormals, infinities
+// and NaNs on the way in; results outside the normal float range on the way out).  After a plain test the compiler
+// predicates the conversion instruction, and a predicated-off F2F still takes its turn in the FP64 pipe: the mixed
+// filter sweeps spent 3.8 FP64 instructions a point and field, 1.4 of them its own additions.  Results are the
+// instruction's, bit for bit (checked on the device by ati_check_conversions).
+template <int K>
+__device__ __forceinline__ void narrow_all(const double (&v)[K], float (&o)[K]) {
+  bool odd = false;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const unsigned hi = (unsigned)__double2hiint(v[k]), lo = (unsigned)__double2loint(v[k]);
+    odd |= (hi & 0x7fffffffu) - (897u << 20) >= (254u << 20);
+    const unsigned m = __funnelshift_l(lo, hi, 3);  // the significand's top 23 bits under the exponent's low bits
+    const unsigned up = (lo & 0x1fffffffu) + 0x0fffffffu + (m & 1u);  // bit 29: round up (ties to even)
+    o[k] = __uint_as_float((m - (896u << 23) + (up >> 29)) | (hi & 0x80000000u));
+  }
+  if (odd) {
+    keep_branch();
+#pragma unroll
+    for (int k = 0; k < K; k++) o[k] = (float)v[k];
+  }
+}
+template <int K>
+__device__ __forceinline__ void widen_all(const float (&v)[K], double (&o)[K]) {
+  bool odd = false;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const unsigned u = __float_as_uint(v[k]), a = u & 0x7fffffffu;
+    odd |= a - 0x00800000u >= 0x7f000000u;
+    o[k] = __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + (896u << 20))), (int)(u << 29));
+  }
+  if (odd) {
+    keep_branch();
+#pragma unroll
+    for (int k = 0; k < K; k++) o[k] = (double)v[k];
+  }
+}
+
 // conversion between the engine types: FP32 -> FP64 on the integer pipes.  The
 // other direction stays with the conversion instruction here: rounding takes some
 // 15 integer operations and branches, slower in the line sweeps' load loops than

@@ -711,6 +711,12 @@ __global__ void __launch_bounds__(XC_NL) k_sweep_xc(SweepArgs<TI, TO, TC> a) {
   }
 }
 
+// the scheme's coefficients into shared memory by all threads' asynchronous copies (the caller commits and waits)
+__device__ __forceinline__ void stage_coef(Coef<float> &dst, const Coef<float> *src) {
+  for (int k = threadIdx.x; k < (int)(sizeof(Coef<float>) / sizeof(float)); k += blockDim.x)
+    cp_async<4>(reinterpret_cast<float *>(&dst) + k, reinterpret_cast<const float *>(src) + k);
+}
+
 // ---------------------------------------------------------------------------
 // Segmented line solves (mixed path, FP32 arithmetic).  A CTA takes SEG_LINES
 // consecutive lines of one block and one field and stages them whole in
@@ -728,11 +734,24 @@ __global__ void __launch_bounds__(XC_NL) k_sweep_xc(SweepArgs<TI, TO, TC> a) {
 // once, with no forward-value scratch.  The results differ from the
 // sequential solve by rounding only, and depend on the line length alone.
 // ---------------------------------------------------------------------------
+// What bounds it, at 24.6 M points (traffic floor 131 us a derivative launch of 4.5 fields, 292 us a filter): the
+// instructions of the recurrences (a third of them loads and stores of shared memory and tables) and, in the
+// filter, the FP64 pipe and the latency of its FP64 loads.  Measured there, us a launch, before and after the steps
+// named:
+//   - coefficients and block fields loaded under the staging's latency instead of at the line ends, where every
+//     CTA waited for them with L1 misses one after the other, and factors of two passes in flight (unroll 2):
+//     xi derivative 401 -> 397, eta 319 -> 295, zeta (with its tiles copied by the threads instead of TMA, whose
+//     one-thread issue of 128-byte rows, a plane apart, took longer than the solve) 341 -> 251;
+//   - the filter's FP64 conversions with a real branch around the conversion instruction (narrow_all, widen_all:
+//     4 -> 1.4 FP64 instructions a point), eight loads in flight in the staging and the next pass's inputs read
+//     before this pass's stores: filters xi 908 -> 715, eta 834 -> 594, zeta 762 -> 652 us.
+// Registers: 64, which the derivatives' occupancy (28 warps an SM) needs; the zeta filter, two warps a CTA with two
+// outputs, takes 80 (at 64 it spills: 691 us; the eta filter at 80 loses a CTA of five warps: 744 us).
 // TMA (eta and zeta derivative sweeps over FP32 inputs, blocks whose geometry a tensor map can describe): the
 // tile of each line group comes in as one tensor copy, [point][line] rows of SEG_LINES floats; eta tiles then
 // hold lines of one grid row only (the work queue's eta tiles start at row starts and multiples of 32 points)
 template <int NN, bool FILT, bool TMA, typename TI, typename TO>
-__global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, TO, float> a, const float *rtab,
+__global__ void __maxnreg__(FILT && NN == 3 ? 80 : 64) k_sweep_seg(SweepArgs<TI, TO, float> a, const float *rtab,
                                                                   int groups) {
   static_assert(!TMA || (NN != 1 && std::is_same<TI, float>::value), "TMA staging: eta/zeta lines of FP32 inputs");
   extern __shared__ __align__(16) unsigned char seg_smem[];
@@ -744,6 +763,13 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
   const int nwarp = (int)(blockDim.x >> 5);
   const LTile LT = a.lt[blockIdx.x];
   const BlockDev &B = a.blk[LT.b];
+  // what the later phases read of the block and the scheme is loaded here, under the staging's latency: the
+  // block's fields in registers, the coefficients in shared memory
+  __shared__ Coef<float> C;
+  stage_coef(C, a.cf);
+  const int ndf[2] = {B.ndf[0][NN], B.ndf[1][NN]};
+  const bool self[2] = {!FILT && B.nbc[0][NN] == 45 && B.ncd[0][NN] == LT.b, !FILT && B.nbc[1][NN] == 45 && B.ncd[1][NN] == LT.b};
+  const int64_t face0 = B.face_off[NN], fac0 = B.fac_off[NN];
   const int f = blockIdx.y;
   const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
   const int L = NN == 1 ? B.lxi + 1 : (NN == 2 ? B.let + 1 : B.lze + 1);
@@ -797,10 +823,32 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       if (!tma_ok && lane == 0) atomicOr(&a.scal[B.cs].flag, FLAG_TIMEOUT);
     }
   }
-  auto stage = [&](float *dst, const TI *src) {
-    if constexpr (ASYNC) cp_async<4>(dst, src);
-    else *dst = cvt_in<TI, float>(__ldg(src), ofs);
+  // rows of a line, K at a time: dst and src walk by dd and ds
+  bool shifted = false;  // (a test of the bits: the compiler repeats it per batch, and an FP64 compare takes that pipe)
+  if constexpr (!ASYNC) shifted = (__double_as_longlong(ofs) << 1) != 0;
+  auto stage = [&](float *dst, int dd, const TI *src, int64_t ds, auto count) {
+    constexpr int K = decltype(count)::value;
+    if constexpr (ASYNC) {
+#pragma unroll
+      for (int k = 0; k < K; k++) cp_async<4>(dst + k * dd, src + k * ds);
+    } else {
+      TI v[K];
+      float x[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) v[k] = __ldg(src + k * ds);
+      if (shifted) {  // (x - 0 is x: no subtraction for offset-free fields)
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] -= ofs;
+      }
+      narrow_all<K>(v, x);
+#pragma unroll
+      for (int k = 0; k < K; k++) dst[k * dd] = x[k];
+    }
   };
+  // (FP64 rows wait for their loads: eight at a time, then four)
+  constexpr std::integral_constant<int, 8> eight{};
+  constexpr std::integral_constant<int, 4> four{};
+  constexpr std::integral_constant<int, 1> one{};
   if constexpr (TMA) {
     // (staged by the tensor copy above)
   } else if constexpr (NN == 1) {
@@ -809,8 +857,11 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
     for (int ln = wl; ln < nl; ln += gsz) {
       const TI *src = src0 + (int64_t)ln * L + lane;
       float *dst = tile + lane * RS + ln;
-#pragma unroll 4
-      for (int i = lane; i < L; i += 32, src += 32, dst += 32 * RS) stage(dst, src);
+      int i = lane;
+      if (!ASYNC)
+        for (; i + 224 < L; i += 256, src += 256, dst += 256 * RS) stage(dst, 32 * RS, src, 32, eight);
+      for (; i + 96 < L; i += 128, src += 128, dst += 128 * RS) stage(dst, 32 * RS, src, 32, four);
+      for (; i < L; i += 32, src += 32, dst += 32 * RS) stage(dst, 0, src, 0, one);
     }
   } else {
     // consecutive eta/zeta lines are consecutive points of a row: a warp copies one row at a time
@@ -818,14 +869,15 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       const TI *src = in + base + (int64_t)wl * stride;
       const int64_t step = (int64_t)gsz * stride;
       float *dst = tile + wl * RS + lane;
-#pragma unroll 4
-      for (int i = wl; i < L; i += gsz, src += step, dst += gsz * RS) stage(dst, src);
+      int i = wl;
+      if (!ASYNC)
+        for (; i + 7 * gsz < L; i += 8 * gsz, src += 8 * step, dst += 8 * gsz * RS) stage(dst, gsz * RS, src, step, eight);
+      for (; i + 3 * gsz < L; i += 4 * gsz, src += 4 * step, dst += 4 * gsz * RS) stage(dst, gsz * RS, src, step, four);
+      for (; i < L; i += gsz, src += step, dst += gsz * RS) stage(dst, 0, src, 0, one);
     }
   }
-  if constexpr (ASYNC) {
-    cp_async_commit();
-    cp_async_wait<0>();
-  }
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
 
   const int S = seg_count(L);
@@ -833,10 +885,9 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
   const int s0 = seg_start(wl, L, S), s1 = seg_start(wl + 1, L, S);
   float *col = tile + lane;
   // the block's row table, SEG_RT floats per row (layout at SEG_RT)
-  const float *rt = rtab + (int64_t)B.fac_off[NN] * SEG_RT;
+  const float *rt = rtab + fac0 * SEG_RT;
   auto row = [&](int i) { return rt + i * SEG_RT; };
   // interior stencil weights in registers (loads from the coefficient struct could not move past the stores)
-  const Coef<float> &C = *a.cf;
   const float k1 = FILT ? C.fa : C.aa, k2 = FILT ? C.fb : C.ab, k3 = FILT ? C.fc : C.ac;
   auto rhs = [&](float x0, float x1, float x2, float x3, float x4, float x5, float x6) {
     if (!FILT) return k1 * (x4 - x2) + k2 * (x5 - x1) + k3 * (x6 - x0);
@@ -856,7 +907,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       // is staged: the sums of k_mpigo (src/Subroutines3D.f90:16-80) in its operation order, skipping the shared
       // point.  (The filter's closures come from the state before its first direction, src/Main3D.f90:555-561,
       // so a filter sweep, which sees the state after the earlier directions, reads them from recv.)
-      const float *rcv = a.recv + f * a.recv_fs + B.face_off[NN] * 6;
+      const float *rcv = a.recv + f * a.recv_fs + face0 * 6;
       const int64_t nbs = B.nbsize[NN];
       constexpr int nt = FILT ? 1 : 0, mp = FILT ? LMF : LMD;
       auto closure = [&](int r0, int dir, float *o) {
@@ -871,11 +922,11 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       };
       float rl[6];
       for (int ip = 0; ip <= 1; ip++) {
-        if (B.ndf[ip][NN] != 1) continue;
-        if (!FILT && B.nbc[ip][NN] == 45 && B.ncd[ip][NN] == LT.b) closure(ip == 0 ? L - 2 : 1, ip == 0 ? -1 : 1, rl + 3 * ip);
+        if (ndf[ip] != 1) continue;
+        if (self[ip]) closure(ip == 0 ? L - 2 : 1, ip == 0 ? -1 : 1, rl + 3 * ip);
         else for (int q = 0; q < 3; q++) rl[3 * ip + q] = rcv[jk + nbs * (3 * ip + q)];
       }
-      line_ends<FILT, float>(C, L, B.ndf[0][NN], B.ndf[1][NN], rl, 1, 0, sld, sbs0, sbs1, sbs2, sbe0, sbe1, sbe2);
+      line_ends<FILT, float>(C, L, ndf[0], ndf[1], rl, 1, 0, sld, sbs0, sbs1, sbs2, sbe0, sbe1, sbe2);
     }
     if (ilo < ihi) {
       a0 = sld(ilo - 3); a1 = sld(ilo - 2); a2 = sld(ilo - 1); a3 = sld(ilo); a4 = sld(ilo + 1); a5 = sld(ilo + 2);
@@ -904,6 +955,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       auto l2 = [](const float *t) { return __ldg(reinterpret_cast<const float2 *>(t)); };
       // each pass loads the next pass's factors first (rows past the block read the table's padding)
       float2 m0 = l2(tr), m1 = l2(tr + SEG_RT), m2 = l2(tr + 2 * SEG_RT), m3 = l2(tr + 3 * SEG_RT);
+#pragma unroll (FILT && NN == 3 ? 1 : 2)
       for (; i + 3 < iown; i += 4, pc += 4 * RS, tr += 4 * SEG_RT) {
         const float b0 = pc[3 * RS], b1 = pc[4 * RS], b2 = pc[5 * RS], b3 = pc[6 * RS];
         const float2 n0 = l2(tr + 4 * SEG_RT), n1 = l2(tr + 5 * SEG_RT), n2 = l2(tr + 6 * SEG_RT);
@@ -952,9 +1004,40 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
   }
   TO *out = a.io.out + f * a.io.out_fs;
   TO *out2 = FILT && a.io.out2 ? a.io.out2 + f * a.io.out_fs : nullptr;  // (a derivative has one output)
-  float *drv = (!FILT && a.io.drva) ? a.drva + B.face_off[NN] * 10 : nullptr;
+  float *drv = (!FILT && a.io.drva) ? a.drva + face0 * 10 : nullptr;
   const int64_t nbs = B.nbsize[NN];
   const int m = a.io.m0 + f;
+  // K results at po, po + ds, ...: the filter adds them to its input (rr = rr + sb, src/Subroutines3D.f90:200-202),
+  // read here before any of the K rows is stored
+  auto fetch = [&](const TI *pi, int64_t ds, auto &q) {  // the filter's inputs of K rows
+    if constexpr (FILT) {
+#pragma unroll
+      for (int k = 0; k < (int)(sizeof(q) / sizeof(q[0])); k++) q[k] = pi[k * ds];
+    }
+  };
+  auto put = [&](TO *po, TO *po2, const auto &q, int64_t ds, const auto &v) {
+    constexpr int K = (int)(sizeof(v) / sizeof(v[0]));
+    TO r[K];
+    if constexpr (FILT) {
+      TI x[K];
+      if constexpr (std::is_same<TI, float>::value) {
+#pragma unroll
+        for (int k = 0; k < K; k++) x[k] = v[k];
+      } else {
+        widen_all<K>(v, x);
+      }
+#pragma unroll
+      for (int k = 0; k < K; k++) r[k] = (TO)(q[k] + x[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < K; k++) r[k] = (TO)v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      po[k * ds] = r[k];
+      if (out2) po2[k * ds] = r[k];
+    }
+  };
   // 5. the segment's forward values, then its back substitution from zero values beyond its end; with one
   // segment that gives the results, which eta/zeta lines write straight to DRAM (a warp writes a row)
   if (act) {
@@ -975,35 +1058,53 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       auto bwd = [&](float *c, const float4 g, const float c4) {
         const float v = *c + g.x * x.x + g.y * x.y;
         const float q = g.z * v - g.w * q1 - c4 * q2;
-        if constexpr (D) {
-          TO r;
-          if (FILT) r = (TO)(*pi + cvt<TI>(q));  // rr = rr + sb (src/Subroutines3D.f90:200-202)
-          else r = (TO)q;
-          *po = r;
-          po -= stride;
-          if (out2) { *po2 = r; po2 -= stride; }
-          if (FILT) pi -= stride;
-        } else {
-          *c = q;
-        }
+        if constexpr (!D) *c = q;
         q2 = q1; q1 = q;
+        return q;
       };
+      auto emit = [&](const auto &v, const auto &q) {  // D: the results of the pass, the last row first
+        put(po, po2, q, -stride, v);
+        const int64_t o = (int64_t)(sizeof(v) / sizeof(v[0])) * stride;
+        po -= o;
+        if (out2) po2 -= o;
+      };
+      auto next = [&](auto &q) {  // the filter's inputs of the next rows, a pass ahead of their use
+        fetch(pi, -stride, q);
+        if (FILT) pi -= (int64_t)(sizeof(q) / sizeof(q[0])) * stride;
+      };
+      TI qa[4] = {0, 0, 0, 0}, qb[4] = {0, 0, 0, 0};
+      if (D && i - 3 >= s0) next(qa);
       float4 g0 = l4(tr), g1 = l4(tr - SEG_RT), g2 = l4(tr - 2 * SEG_RT), g3 = l4(tr - 3 * SEG_RT);
       float k0 = l1(tr), k1 = l1(tr - SEG_RT), k2 = l1(tr - 2 * SEG_RT), k3 = l1(tr - 3 * SEG_RT);
+#pragma unroll (FILT && NN == 3 ? 1 : 2)
       for (; i - 3 >= s0; i -= 4, pc -= 4 * RS, tr -= 4 * SEG_RT) {
         // the next pass's rows (rows before the block read the table's padding)
         const float4 h0 = l4(tr - 4 * SEG_RT), h1 = l4(tr - 5 * SEG_RT), h2 = l4(tr - 6 * SEG_RT);
         const float4 h3 = l4(tr - 7 * SEG_RT);
         const float j0 = l1(tr - 4 * SEG_RT), j1 = l1(tr - 5 * SEG_RT), j2 = l1(tr - 6 * SEG_RT);
         const float j3 = l1(tr - 7 * SEG_RT);
-        bwd(pc, g0, k0);
-        bwd(pc - RS, g1, k1);
-        bwd(pc - 2 * RS, g2, k2);
-        bwd(pc - 3 * RS, g3, k3);
+        float v[4];
+        v[0] = bwd(pc, g0, k0);
+        v[1] = bwd(pc - RS, g1, k1);
+        v[2] = bwd(pc - 2 * RS, g2, k2);
+        v[3] = bwd(pc - 3 * RS, g3, k3);
+        if constexpr (D) {
+          if (i - 7 >= s0) next(qb);
+          emit(v, qa);
+#pragma unroll
+          for (int k = 0; k < 4; k++) qa[k] = qb[k];
+        }
         g0 = h0; g1 = h1; g2 = h2; g3 = h3;
         k0 = j0; k1 = j1; k2 = j2; k3 = j3;
       }
-      for (; i >= s0; i--, pc -= RS, tr -= SEG_RT) bwd(pc, l4(tr), l1(tr));
+      for (; i >= s0; i--, pc -= RS, tr -= SEG_RT) {
+        const float v[1] = {bwd(pc, l4(tr), l1(tr))};
+        if constexpr (D) {
+          TI q[1];
+          next(q);
+          emit(v, q);
+        }
+      }
     };
     if (!multi && NN != 1) {
       sweep(std::true_type{});
@@ -1054,6 +1155,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
       const float *tr = row(i) + 8;
       float2 e0 = l2(tr), e1 = l2(tr + SEG_RT), e2 = l2(tr + 2 * SEG_RT), e3 = l2(tr + 3 * SEG_RT);
       if constexpr (NN == 1) {
+#pragma unroll 2
         for (; i + 3 < s1; i += 4, pc += 4 * RS, tr += 4 * SEG_RT) {
           const float2 f0 = l2(tr + 4 * SEG_RT), f1 = l2(tr + 5 * SEG_RT), f2 = l2(tr + 6 * SEG_RT);
           const float2 f3 = l2(tr + 7 * SEG_RT);
@@ -1068,49 +1170,64 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
         TO *po = out + o;
         TO *po2 = out2 ? out2 + o : nullptr;
         const TI *pi = in + o;
-        auto put = [&](float v) {
-          TO r;
-          if (FILT) r = (TO)(*pi + cvt<TI>(v));  // rr = rr + sb (src/Subroutines3D.f90:200-202)
-          else r = (TO)v;
-          *po = r;
-          po += stride;
-          if (out2) { *po2 = r; po2 += stride; }
-          if (FILT) pi += stride;
+        auto emit = [&](const auto &v, const auto &q) {
+          put(po, po2, q, stride, v);
+          const int64_t o = (int64_t)(sizeof(v) / sizeof(v[0])) * stride;
+          po += o;
+          if (out2) po2 += o;
         };
+        auto next = [&](auto &q) {
+          fetch(pi, stride, q);
+          if (FILT) pi += (int64_t)(sizeof(q) / sizeof(q[0])) * stride;
+        };
+        TI qa[4] = {0, 0, 0, 0}, qb[4] = {0, 0, 0, 0};
+        if (i + 3 < s1) next(qa);
+#pragma unroll (FILT && NN == 3 ? 1 : 2)
         for (; i + 3 < s1; i += 4, pc += 4 * RS, tr += 4 * SEG_RT) {
           const float2 f0 = l2(tr + 4 * SEG_RT), f1 = l2(tr + 5 * SEG_RT), f2 = l2(tr + 6 * SEG_RT);
           const float2 f3 = l2(tr + 7 * SEG_RT);
-          const float r0 = fg(pc, e0), r1 = fg(pc + RS, e1), r2 = fg(pc + 2 * RS, e2), r3 = fg(pc + 3 * RS, e3);
-          put(r0); put(r1); put(r2); put(r3);
+          const float r[4] = {fg(pc, e0), fg(pc + RS, e1), fg(pc + 2 * RS, e2), fg(pc + 3 * RS, e3)};
+          if (i + 7 < s1) next(qb);
+          emit(r, qa);
+#pragma unroll
+          for (int k = 0; k < 4; k++) qa[k] = qb[k];
           e0 = f0; e1 = f1; e2 = f2; e3 = f3;
         }
-        for (; i < s1; i++, pc += RS, tr += SEG_RT) put(fv(pc, tr));
+        for (; i < s1; i++, pc += RS, tr += SEG_RT) {
+          const float r[1] = {fv(pc, tr)};
+          TI q[1];
+          next(q);
+          emit(r, q);
+        }
       }
     }
   }
   if constexpr (NN == 1) {
     __syncthreads();
     const int64_t o0 = B.off + (int64_t)t0 * L;
-    auto wr = [&](int64_t p, float v, TI qin) {
-      TO r;
-      if (FILT) r = (TO)(qin + cvt<TI>(v));  // rr = rr + sb (src/Subroutines3D.f90:200-202)
-      else r = (TO)v;
-      out[p] = r;
-      if (out2) out2[p] = r;
-    };
     for (int ln = wl; ln < nl; ln += gsz) {
       const int64_t lb = o0 + (int64_t)ln * L;
+      auto emit = [&](int i, const auto &v) {
+        TI q[sizeof(v) / sizeof(v[0])];
+        fetch(in + lb + i, 32, q);
+        put(out + lb + i, out2 + lb + i, q, 32, v);
+      };
       int i = lane;
-      // four points a pass, their inputs read before any of them is stored (the filter runs in place)
-      for (; i + 96 < L; i += 128) {
-        TI q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-        if (FILT) { q0 = in[lb + i]; q1 = in[lb + i + 32]; q2 = in[lb + i + 64]; q3 = in[lb + i + 96]; }
-        wr(lb + i, tile[i * RS + ln], q0);
-        wr(lb + i + 32, tile[(i + 32) * RS + ln], q1);
-        wr(lb + i + 64, tile[(i + 64) * RS + ln], q2);
-        wr(lb + i + 96, tile[(i + 96) * RS + ln], q3);
+      auto rows = [&](auto count) {
+        constexpr int K = decltype(count)::value;
+        for (; i + 32 * (K - 1) < L; i += 32 * K) {
+          float v[K];
+#pragma unroll
+          for (int k = 0; k < K; k++) v[k] = tile[(i + 32 * k) * RS + ln];
+          emit(i, v);
+        }
+      };
+      if (FILT) rows(eight);
+      rows(four);
+      for (; i < L; i += 32) {
+        const float v[1] = {tile[i * RS + ln]};
+        emit(i, v);
       }
-      for (; i < L; i += 32) wr(lb + i, tile[i * RS + ln], FILT ? in[lb + i] : (TI)0);
     }
   }
   if constexpr (TMA) {
@@ -1137,93 +1254,68 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_seg(SweepArgs<TI, 
 // rows, as in k_sweep_seg); with TMA each half comes in as one tensor copy, both
 // counted on one mbarrier.
 // ---------------------------------------------------------------------------
-// ADJ: the second half's line l lies SEG_LINES points after the first half's (zeta lines, and eta lines in row
-// tiles): its results are stored at a fixed offset from the first half's, through one walking pointer.
-template <int NN, bool TMA, bool ADJ>
+// The second half's line l lies SEG_LINES points after the first half's: its results are stored at a fixed offset
+// from the first half's, through one walking pointer.
+template <int NN>
 __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<float, float, float> a, const float *rtab,
                                                                    int single) {
-  static_assert(!ADJ || NN != 1, "adjacent halves: eta/zeta lines");
   extern __shared__ __align__(16) unsigned char seg_smem[];
-  constexpr int RS = TMA ? SEG_LINES : SEG_LINES + 1;
+  constexpr int RS = SEG_LINES;
   __shared__ uint64_t tbar;
   const int nwarp = (int)(blockDim.x >> 5);
   const LTile LT = a.lt[single ? blockIdx.x : 2 * blockIdx.x];
   const BlockDev &B = a.blk[LT.b];
+  // what the later phases read of the block and the scheme is loaded here, under the staging's latency: the
+  // block's fields in registers, the coefficients in shared memory
+  __shared__ Coef<float> C;
+  stage_coef(C, a.cf);
+  const int ndf[2] = {B.ndf[0][NN], B.ndf[1][NN]};
+  const bool self[2] = {B.nbc[0][NN] == 45 && B.ncd[0][NN] == LT.b, B.nbc[1][NN] == 45 && B.ncd[1][NN] == LT.b};
+  const int64_t face0 = B.face_off[NN], fac0 = B.fac_off[NN];
   const int f = blockIdx.y;
   const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
   const int nx = B.lxi + 1, ny = B.let + 1;
-  const int L = NN == 1 ? nx : (NN == 2 ? ny : B.lze + 1);
+  const int L = NN == 2 ? ny : B.lze + 1;
   const int T0 = LT.t0;
   const int64_t nbs = B.nbsize[NN];
   // lines of each half (none past the block's lines or, for eta row tiles, past the grid row)
-  const int lim = T0 >= nbs ? 0 : ((NN == 2 && a.rowtiles) ? nx - T0 % nx : (int)(nbs - T0));
+  const int lim = T0 >= nbs ? 0 : (NN == 2 ? nx - T0 % nx : (int)(nbs - T0));
   const int nl0 = max(0, min(SEG_LINES, lim)), nl1 = max(0, min(SEG_LINES, lim - SEG_LINES));
   const int HS = L * RS;  // offset of the second half's tile
-  float *tiles;
-  if constexpr (TMA) {
-    const uint32_t pad = (128u - (smem_u32(seg_smem) & 127u)) & 127u;
-    tiles = reinterpret_cast<float *>(seg_smem + pad);
-  } else {
-    tiles = reinterpret_cast<float *>(seg_smem + (size_t)nwarp * SEG_LINES * 2 * sizeof(float4));
-  }
+  float *tiles = reinterpret_cast<float *>(seg_smem + ((128u - (smem_u32(seg_smem) & 127u)) & 127u));
   // [segment][lane] values a segment passes on / receives, both halves' lines in one float4
-  float4 *cf = TMA ? reinterpret_cast<float4 *>(tiles + 2 * (int64_t)HS) : reinterpret_cast<float4 *>(seg_smem);
+  float4 *cf = reinterpret_cast<float4 *>(tiles + 2 * (int64_t)HS);
   float4 *cx = cf + nwarp * SEG_LINES;
-  const int64_t stride = NN == 1 ? 1 : (NN == 2 ? (int64_t)nx : (int64_t)nx * ny);
+  const int64_t stride = NN == 2 ? (int64_t)nx : (int64_t)nx * ny;
   int64_t base0 = 0, base1 = 0, sdum = 0;
   int jk0 = 0, jk1 = 0, Lg = 0;
   line_geom<NN>(B, T0 + lane, base0, sdum, jk0, Lg);
   line_geom<NN>(B, T0 + SEG_LINES + lane, base1, sdum, jk1, Lg);
-  const float *in = a.io.in + f * a.io.in_fs;
 
   // 1. stage both halves
   bool tma_ok = true;
-  if constexpr (TMA) {
-    if (threadIdx.x == 0) {
-      mbar_init(&tbar, 1);
-      fence_mbar_init();
-    }
-    __syncthreads();
-    if (nl0 > 0) {
-      if (threadIdx.x == 0) {
-        const TmaMap *tm = a.tmap + LT.b;
-        tmap_acquire(tm);
-        mbar_expect_tx(&tbar, (uint32_t)(L * SEG_LINES * sizeof(float)) * (nl1 > 0 ? 2u : 1u));
-        for (int hh = 0; hh < 2; hh++) {
-          if (hh == 1 && nl1 == 0) break;
-          const int t0 = T0 + hh * SEG_LINES;
-          if constexpr (NN == 2) tma_load_4d(tiles + hh * HS, tm, t0 % nx, 0, t0 / nx, f, &tbar);
-          else tma_load_3d(tiles + hh * HS, tm, t0, 0, f, &tbar);
-        }
-      }
-      tma_ok = mbar_wait_bounded(&tbar, 0);
-      if (!tma_ok && lane == 0) atomicOr(&a.scal[B.cs].flag, FLAG_TIMEOUT);
-    }
-  } else {
-#pragma unroll
-    for (int hh = 0; hh < 2; hh++) {
-      const int nl = hh ? nl1 : nl0;
-      float *tile = tiles + hh * HS;
-      if constexpr (NN == 1) {
-        // xi lines are contiguous: a warp copies one line at a time, lanes along the line
-        const float *src0 = in + B.off + (int64_t)(T0 + hh * SEG_LINES) * L;
-        for (int ln = w; ln < nl; ln += nwarp) {
-          const float *src = src0 + (int64_t)ln * L + lane;
-          float *dst = tile + lane * RS + ln;
-#pragma unroll 4
-          for (int i = lane; i < L; i += 32, src += 32, dst += 32 * RS) cp_async<4>(dst, src);
-        }
-      } else if (lane < nl) {
-        // consecutive eta/zeta lines are consecutive points of a row: a warp copies one row at a time
-        const float *src = in + (hh ? base1 : base0) + (int64_t)w * stride;
-        float *dst = tile + w * RS + lane;
-#pragma unroll 4
-        for (int i = w; i < L; i += nwarp, src += nwarp * stride, dst += nwarp * RS) cp_async<4>(dst, src);
-      }
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
+  if (threadIdx.x == 0) {
+    mbar_init(&tbar, 1);
+    fence_mbar_init();
   }
+  __syncthreads();
+  if (nl0 > 0) {
+    if (threadIdx.x == 0) {
+      const TmaMap *tm = a.tmap + LT.b;
+      tmap_acquire(tm);
+      mbar_expect_tx(&tbar, (uint32_t)(L * SEG_LINES * sizeof(float)) * (nl1 > 0 ? 2u : 1u));
+      for (int hh = 0; hh < 2; hh++) {
+        if (hh == 1 && nl1 == 0) break;
+        const int t0 = T0 + hh * SEG_LINES;
+        if constexpr (NN == 2) tma_load_4d(tiles + hh * HS, tm, t0 % nx, 0, t0 / nx, f, &tbar);
+        else tma_load_3d(tiles + hh * HS, tm, t0, 0, f, &tbar);
+      }
+    }
+    tma_ok = mbar_wait_bounded(&tbar, 0);
+    if (!tma_ok && lane == 0) atomicOr(&a.scal[B.cs].flag, FLAG_TIMEOUT);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
 
   const int S = seg_count(L);
@@ -1232,9 +1324,8 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
   const bool act = act0;
   const int s0 = seg_start(w, L, S), s1 = seg_start(w + 1, L, S);
   float *col = tiles + lane;  // half 0; half 1 at col + HS
-  const float *rt = rtab + (int64_t)B.fac_off[NN] * SEG_RT;
+  const float *rt = rtab + fac0 * SEG_RT;
   auto row = [&](int i) { return rt + i * SEG_RT; };
-  const Coef<float> &C = *a.cf;
   const float k1 = C.aa, k2 = C.ab, k3 = C.ac;
   auto rhs = [&](float x0, float x1, float x2, float x3, float x4, float x5, float x6) {
     return k1 * (x4 - x2) + k2 * (x5 - x1) + k3 * (x6 - x0);
@@ -1251,7 +1342,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
       auto sld = [&](int i) { return ch[i * RS]; };
       if ((hh == 0 || act1) && (w == 0 || w == S - 1)) {
         const int jk = hh ? jk1 : jk0;
-        const float *rcv = a.recv + f * a.recv_fs + B.face_off[NN] * 6;
+        const float *rcv = a.recv + f * a.recv_fs + face0 * 6;
         auto closure = [&](int r0, int dir, float *o) {
           float c0 = 0, c1 = 0, sap0 = 0;
           for (int i = 0; i <= LMD; i++) {
@@ -1264,11 +1355,11 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
         };
         float rl[6];
         for (int ip = 0; ip <= 1; ip++) {
-          if (B.ndf[ip][NN] != 1) continue;
-          if (B.nbc[ip][NN] == 45 && B.ncd[ip][NN] == LT.b) closure(ip == 0 ? L - 2 : 1, ip == 0 ? -1 : 1, rl + 3 * ip);
+          if (ndf[ip] != 1) continue;
+          if (self[ip]) closure(ip == 0 ? L - 2 : 1, ip == 0 ? -1 : 1, rl + 3 * ip);
           else for (int q = 0; q < 3; q++) rl[3 * ip + q] = rcv[jk + nbs * (3 * ip + q)];
         }
-        line_ends<false, float>(C, L, B.ndf[0][NN], B.ndf[1][NN], rl, 1, 0, sld, sbs0[hh], sbs1[hh], sbs2[hh],
+        line_ends<false, float>(C, L, ndf[0], ndf[1], rl, 1, 0, sld, sbs0[hh], sbs1[hh], sbs2[hh],
                                 sbe0[hh], sbe1[hh], sbe2[hh]);
       }
       if (ilo < ihi) {
@@ -1370,7 +1461,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
     __syncthreads();
   }
   float *out = a.io.out + f * a.io.out_fs;
-  float *drv = a.io.drva ? a.drva + B.face_off[NN] * 10 : nullptr;
+  float *drv = a.io.drva ? a.drva + face0 * 10 : nullptr;
   const int m = a.io.m0 + f;
   // 5. the segment's forward values, then its back substitution from zero values beyond its end; with one
   // segment that gives the results, which eta/zeta lines write straight to DRAM (a warp writes a row)
@@ -1381,7 +1472,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
     int i = s1 - 1;
     float *pc = col + i * RS;
     const float *tr = row(i);
-    float *po0 = out + base0 + (int64_t)i * stride, *po1 = out + base1 + (int64_t)i * stride;
+    float *po0 = out + base0 + (int64_t)i * stride;
     auto sweep = [&](auto direct) {
       constexpr bool D = decltype(direct)::value;
       auto l4 = [](const float *t) { return __ldg(reinterpret_cast<const float4 *>(t + 4)); };
@@ -1395,12 +1486,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
         }
         if constexpr (D) {
           *po0 = q[0];
-          if constexpr (ADJ) {
-            if (act1) po0[SEG_LINES] = q[1];
-          } else {
-            if (act1) *po1 = q[1];
-            po1 -= stride;
-          }
+          if (act1) po0[SEG_LINES] = q[1];
           po0 -= stride;
         } else {
           c[0] = q[0];
@@ -1425,7 +1511,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
       }
       for (; i >= s0; i--, pc -= RS, tr -= SEG_RT) bwd(pc, l4(tr), l1(tr));
     };
-    if (!multi && NN != 1) {
+    if (!multi) {
       sweep(std::true_type{});
       if (drv) {
         drv[jk0 + nbs * ((m - 1) + 5 * 0)] = q1[0];  // drva(jk,m,0) = sb(is): row 0, the last one solved
@@ -1437,16 +1523,7 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
       }
     } else {
       sweep(std::false_type{});
-      if (multi) {
-        cf[w * SEG_LINES + lane] = make_float4(q1[0], q2[0], q1[1], q2[1]);  // rows s0, s0+1
-      } else if (drv) {
-        drv[jk0 + nbs * ((m - 1) + 5 * 0)] = col[0];
-        drv[jk0 + nbs * ((m - 1) + 5 * 1)] = col[(L - 1) * RS];
-        if (act1) {
-          drv[jk1 + nbs * ((m - 1) + 5 * 0)] = col[HS];
-          drv[jk1 + nbs * ((m - 1) + 5 * 1)] = col[HS + (L - 1) * RS];
-        }
-      }
+      cf[w * SEG_LINES + lane] = make_float4(q1[0], q2[0], q1[1], q2[1]);  // rows s0, s0+1
     }
   }
   if (multi) {
@@ -1494,79 +1571,30 @@ __global__ void __launch_bounds__(SEG_LINES *SEG_MAX) k_sweep_pair(SweepArgs<flo
 #pragma unroll
         for (int hh = 0; hh < 2; hh++) r[hh] = c[hh * HS] + g.x * y[hh].x + g.y * y[hh].y;
       };
-      if constexpr (NN == 1) {
-        for (; i + 3 < s1; i += 4, pc += 4 * RS, tr += 4 * SEG_RT) {
-          const float2 n0 = l2(tr + 4 * SEG_RT), n1 = l2(tr + 5 * SEG_RT), n2 = l2(tr + 6 * SEG_RT);
-          const float2 n3 = l2(tr + 7 * SEG_RT);
-          float r0[2], r1[2], r2[2], r3[2];
-          fg2(pc, e0, r0); fg2(pc + RS, e1, r1); fg2(pc + 2 * RS, e2, r2); fg2(pc + 3 * RS, e3, r3);
-#pragma unroll
-          for (int hh = 0; hh < 2; hh++) {
-            float *q = pc + hh * HS;
-            q[0] = r0[hh]; q[RS] = r1[hh]; q[2 * RS] = r2[hh]; q[3 * RS] = r3[hh];
-          }
-          e0 = n0; e1 = n1; e2 = n2; e3 = n3;
-        }
-        for (; i < s1; i++, pc += RS, tr += SEG_RT) {
-          float r[2];
-          fg2(pc, l2(tr), r);
-          pc[0] = r[0];
-          pc[HS] = r[1];
-        }
-      } else {
-        // walking output pointers: one 64-bit add per row and half
-        float *po0 = out + base0 + (int64_t)i * stride, *po1 = out + base1 + (int64_t)i * stride;
-        auto put = [&](const float r[2]) {
-          *po0 = r[0];
-          if constexpr (ADJ) {
-            if (act1) po0[SEG_LINES] = r[1];
-          } else {
-            if (act1) *po1 = r[1];
-            po1 += stride;
-          }
-          po0 += stride;
-        };
-        for (; i + 3 < s1; i += 4, pc += 4 * RS, tr += 4 * SEG_RT) {
-          const float2 n0 = l2(tr + 4 * SEG_RT), n1 = l2(tr + 5 * SEG_RT), n2 = l2(tr + 6 * SEG_RT);
-          const float2 n3 = l2(tr + 7 * SEG_RT);
-          float r0[2], r1[2], r2[2], r3[2];
-          fg2(pc, e0, r0); fg2(pc + RS, e1, r1); fg2(pc + 2 * RS, e2, r2); fg2(pc + 3 * RS, e3, r3);
-          put(r0); put(r1); put(r2); put(r3);
-          e0 = n0; e1 = n1; e2 = n2; e3 = n3;
-        }
-        for (; i < s1; i++, pc += RS, tr += SEG_RT) {
-          float r[2];
-          fg2(pc, l2(tr), r);
-          put(r);
-        }
+      // a walking output pointer: one 64-bit add per row
+      float *po0 = out + base0 + (int64_t)i * stride;
+      auto put = [&](const float r[2]) {
+        *po0 = r[0];
+        if (act1) po0[SEG_LINES] = r[1];
+        po0 += stride;
+      };
+      for (; i + 3 < s1; i += 4, pc += 4 * RS, tr += 4 * SEG_RT) {
+        const float2 n0 = l2(tr + 4 * SEG_RT), n1 = l2(tr + 5 * SEG_RT), n2 = l2(tr + 6 * SEG_RT);
+        const float2 n3 = l2(tr + 7 * SEG_RT);
+        float r0[2], r1[2], r2[2], r3[2];
+        fg2(pc, e0, r0); fg2(pc + RS, e1, r1); fg2(pc + 2 * RS, e2, r2); fg2(pc + 3 * RS, e3, r3);
+        put(r0); put(r1); put(r2); put(r3);
+        e0 = n0; e1 = n1; e2 = n2; e3 = n3;
+      }
+      for (; i < s1; i++, pc += RS, tr += SEG_RT) {
+        float r[2];
+        fg2(pc, l2(tr), r);
+        put(r);
       }
     }
   }
-  if constexpr (NN == 1) {
-    __syncthreads();
-    // both halves' lines back to DRAM through the tiles, a warp along one line at a time
-#pragma unroll
-    for (int hh = 0; hh < 2; hh++) {
-      const int nl = hh ? nl1 : nl0;
-      const float *tile = tiles + hh * HS;
-      const int64_t o0 = B.off + (int64_t)(T0 + hh * SEG_LINES) * L;
-      for (int ln = w; ln < nl; ln += nwarp) {
-        const int64_t lb = o0 + (int64_t)ln * L;
-        int i = lane;
-        for (; i + 96 < L; i += 128) {
-          out[lb + i] = tile[i * RS + ln];
-          out[lb + i + 32] = tile[(i + 32) * RS + ln];
-          out[lb + i + 64] = tile[(i + 64) * RS + ln];
-          out[lb + i + 96] = tile[(i + 96) * RS + ln];
-        }
-        for (; i < L; i += 32) out[lb + i] = tile[i * RS + ln];
-      }
-    }
-  }
-  if constexpr (TMA) {
-    // a tile copy that did not land in time: wait once more (bounded) before the CTA exits
-    if (!tma_ok) (void)mbar_wait_bounded(&tbar, 0);
-  }
+  // a tile copy that did not land in time: wait once more (bounded) before the CTA exits
+  if (!tma_ok) (void)mbar_wait_bounded(&tbar, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -3121,30 +3149,21 @@ static void sweep_t(const Eng<TC> &e, cudaStream_t st, int nn, bool filt, const 
           // eta/zeta derivative sweeps of an array with tensor maps: tiles staged by TMA
           const int arr = io.in == e.prim ? 0 : (io.in == e.flx + (int64_t)(nn - 1) * e.N ? 1 : -1);
           const bool tma = !filt && nn >= 2 && e.tma[nn] && arr >= 0;
+          if (tma) a.tmap = e.tmaps + (int64_t)(arr * 2 + nn - 2) * e.nblk;
           // paired lines: a CTA solves two groups of lines, lane l line l of each (lines of up to PAIR_MAX_SEG
-          // segments: longer ones would halve the CTAs an SM holds, measured slower)
+          // segments: longer ones would halve the CTAs an SM holds, measured slower).  Without TMA the single-group
+          // kernel is as fast or faster (eta, us a launch, pair and single: 122.8 and 119.7 at 120 points a line,
+          // 66.4 and 65.6 at 91; xi 22.2 and 22.0 at 160).
           const size_t psm = pair_smem_bytes(C.maxlen, G > 1) + 128;
-          if (!filt && e.pairs && seg_count(C.maxlen) <= PAIR_MAX_SEG && psm <= SEG_SMEM_MAX) {
+          if (tma && e.pairs && seg_count(C.maxlen) <= PAIR_MAX_SEG && psm <= SEG_SMEM_MAX) {
             const int single = G > 1 ? 1 : 0;
             const dim3 gp(single ? C.n : C.n / 2, io.nf);
             const int ntp = SEG_LINES * (single ? 1 : seg_count(C.maxlen));
-            const bool adj = nn == 3 || (nn == 2 && e.eta_rowtiles);
-            if (tma) a.tmap = e.tmaps + (int64_t)(arr * 2 + nn - 2) * e.nblk;
-#define ATI_PAIR(D, T, J) k_sweep_pair<D, T, J><<<gp, ntp, psm, st>>>(a, seg, single)
-            if (nn == 1) ATI_PAIR(1, false, false);
-            else if (nn == 2) {
-              if (tma) ATI_PAIR(2, true, true);
-              else if (adj) ATI_PAIR(2, false, true);
-              else ATI_PAIR(2, false, false);
-            } else {
-              if (tma) ATI_PAIR(3, true, true);
-              else ATI_PAIR(3, false, true);
-            }
-#undef ATI_PAIR
+            if (nn == 2) k_sweep_pair<2><<<gp, ntp, psm, st>>>(a, seg, single);
+            else k_sweep_pair<3><<<gp, ntp, psm, st>>>(a, seg, single);
             continue;
           }
           if (tma) {
-            a.tmap = e.tmaps + (int64_t)(arr * 2 + nn - 2) * e.nblk;
             const size_t sm = smem + 128;  // (alignment of the tensor copies' destination)
             if (nn == 2) k_sweep_seg<2, false, true, TI, TO><<<g, nt, sm, st>>>(a, seg, G);
             else k_sweep_seg<3, false, true, TI, TO><<<g, nt, sm, st>>>(a, seg, G);
@@ -3205,12 +3224,8 @@ static cudaError_t seg_attr() {
   if constexpr (std::is_same<TI, float>::value) {
     if (e == cudaSuccess) e = seg_attr_one(k_sweep_seg<2, false, true, TI, TO>);
     if (e == cudaSuccess) e = seg_attr_one(k_sweep_seg<3, false, true, TI, TO>);
-    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<1, false, false>);
-    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<2, false, false>);
-    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<2, false, true>);
-    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<3, false, true>);
-    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<2, true, true>);
-    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<3, true, true>);
+    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<2>);
+    if (e == cudaSuccess) e = seg_attr_one(k_sweep_pair<3>);
   }
   return e;
 }
