@@ -1763,6 +1763,64 @@ __global__ void k_mpigo(const BlockDev *blk, const Coef<TC> *cf, const FaceTask 
     if (const PTile T = (e).pt[t_]; true)
 #define POINT_LOOP(T, g) for (int64_t g = (T).g0 + threadIdx.x; g < (T).g1; g += blockDim.x)
 
+// Groups of consecutive points.  The mixed path's flux and divergence kernels stream some forty planes a point; with one
+// 4-byte access a point and plane they ran at 5 TB/s (staged through shared memory or not), with 8-byte accesses, all of
+// a group's loads in flight before its first result and no shared memory, at 6.9 TB/s.
+// KEEP: planes that later kernels read again; the others are marked for early eviction.
+template <bool KEEP, typename T>
+__device__ __forceinline__ T ld_stream(const T *p) { return KEEP ? __ldg(p) : __ldcs(p); }
+// V consecutive values at p (V x their size aligned)
+template <int V, bool KEEP = false>
+__device__ __forceinline__ void vload(float (&o)[V], const float *p) {
+  if constexpr (V == 1) o[0] = ld_stream<KEEP>(p);
+  else if constexpr (V == 2) { const float2 v = ld_stream<KEEP>(reinterpret_cast<const float2 *>(p)); o[0] = v.x; o[1] = v.y; }
+  else { const float4 v = ld_stream<KEEP>(reinterpret_cast<const float4 *>(p)); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+}
+template <int V, bool KEEP = false>
+__device__ __forceinline__ void vload(double (&o)[V], const double *p) {
+  if constexpr (V == 1) o[0] = ld_stream<KEEP>(p);
+  else {
+#pragma unroll
+    for (int k = 0; k < V; k += 2) {
+      const double2 v = ld_stream<KEEP>(reinterpret_cast<const double2 *>(p + k));
+      o[k] = v.x; o[k + 1] = v.y;
+    }
+  }
+}
+template <int V>
+__device__ __forceinline__ void vstore(double *p, const double (&v)[V]) {
+  if constexpr (V == 1) *p = v[0];
+  else {
+#pragma unroll
+    for (int k = 0; k < V; k += 2) *reinterpret_cast<double2 *>(p + k) = make_double2(v[k], v[k + 1]);
+  }
+}
+template <int V>
+__device__ __forceinline__ void vstore(float *p, const float (&v)[V]) {
+  if constexpr (V == 1) *p = v[0];
+  else if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+  else *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// the points of tile T in groups of V consecutive ones, the first group from a multiple of V; a group at a tile's end
+// may reach into the neighbouring tile's points, which its kernel does not store
+#define GROUP_LOOP(T, g, V) \
+  for (int64_t g = ((T).g0 & ~(int64_t)((V) - 1)) + (V) * (int64_t)threadIdx.x; g < (T).g1; g += (V) * (int64_t)blockDim.x)
+// stores v[c] (planes N apart) at o = plane + g for the group's points that are the tile's own
+template <int V, int C, typename T>
+__device__ __forceinline__ void put_group(T *o, int64_t N, const PTile &t, int64_t g, const T (&v)[C][V]) {
+  if (V == 1 || (g >= t.g0 && g + V <= t.g1)) {
+#pragma unroll
+    for (int c = 0; c < C; c++) vstore<V>(o + c * N, v[c]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      if (g + k >= t.g0 && g + k < t.g1)
+#pragma unroll
+        for (int c = 0; c < C; c++) o[k + c * N] = v[c][k];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Shared-memory staging of the mixed path's streaming kernels.  Each thread
 // copies (cp.async) the input planes of the points it will take STG - 1 points
@@ -2147,7 +2205,7 @@ __device__ __forceinline__ void flux_fast_point(const Eng<double> &e, int64_t N,
 // (src/Main3D.f90:710-766): flx plane (m-1)*3 + (nn-1)
 // (the FP32 kernel streams: five CTAs of 256 threads an SM, at most 51 registers a thread, keep more loads
 // in flight than the 80 registers it would take unbounded; measured 380 -> 296 us a launch on 8.85 M points)
-// (the mixed path's viscous fluxes take the stresses at the point instead: k_flux_staged; the FP64 fast path's run in fixed
+// (the mixed path's viscous fluxes take the stresses at the point instead: k_flux_mixed; the FP64 fast path's run in fixed
 // point, k_flux_fixed, but with the LES terms)
 template <typename R>
 __global__ void __launch_bounds__(256, Freestream<R>::on ? 5 : 1) k_flux(Eng<R> e) {
@@ -2289,149 +2347,162 @@ __global__ void __launch_bounds__(256, 2) k_flux_fixed(const __grid_constant__ E
   }
 }
 
-// the mixed path's viscous fluxes (k_flux with the stresses of k_visc taken at the point), inputs staged:
-// 5 FP64 state planes and 27 FP32 planes a point (metrics 9, derivative planes 12, Jacobian, viscosity,
-// velocity 3, pressure); no stress plane is written or read
-constexpr int FXS_STG = 2, FXS_ND = 5, FXS_NF = 27;
-struct FluxStageIn {
-  const float *f;  // the point's FP32 planes in shared memory, plane stride nt
-  const double *d;
-  int nt;
-  __device__ float at(int p) const { return f[p * nt]; }
-  __device__ float dv(int k) const { return at(9 + k); }
-  __device__ float yac() const { return at(21); }
-  __device__ float mu() const { return at(22); }
-  __device__ float rho() const { return cvt<float>(d[0]); }
-  __device__ float vel(int k) const { return at(23 + k); }
+// The mixed path's viscous fluxes (k_flux with the stresses of k_visc taken at the point): 5 FP64 state planes and 27 FP32
+// planes a point (metrics 9, derivative planes 12, Jacobian, viscosity, velocity 3, pressure) in, 15 FP32 planes out; no
+// stress plane is written or read.  The traffic bounds it (208 B a point: 757 us at 24.6 M points).  Two points a thread
+// where every plane starts on a pair (an even number of points), 128 registers and two CTAs an SM: 742 us, 115 us at
+// 3.6 M and 34 us at 0.9 M points, against 1014, 153 and 45 us with the inputs staged through shared memory by 4-byte
+// asynchronous copies.  One point a thread (odd counts): 838, 125 and 33 us at three CTAs an SM.  Only the derivative
+// planes, which no later kernel reads, are marked for early eviction (all planes: 772 and 31 us, none: 737 and 34 us).
+struct FluxIn {
+  float f[27];
+  float q[7];  // rho, rho u, rho v, rho w, rho E, rho - rho_inf, rho E - rho E_inf
+  __device__ float at(int p) const { return f[p]; }
+  __device__ float dv(int k) const { return f[9 + k]; }
+  __device__ float yac() const { return f[21]; }
+  __device__ float mu() const { return f[22]; }
+  __device__ float rho() const { return q[0]; }
+  __device__ float vel(int k) const { return f[23 + k]; }
 };
-size_t flux_staged_smem(int nt) {
-  return Ring<double, FXS_ND, FXS_STG>::bytes(nt) + Ring<float, FXS_NF, FXS_STG>::bytes(nt);
-}
-
-__global__ void __launch_bounds__(256, 3) k_flux_staged(Eng<float> e) {
-  extern __shared__ __align__(16) unsigned char fxs_smem[];
-  const int nt = blockDim.x;
+template <int V>
+__global__ void __launch_bounds__(256, V == 1 ? 3 : 2) k_flux_mixed(const __grid_constant__ Eng<float> e) {
   const int64_t N = e.N;
-  Ring<double, FXS_ND, FXS_STG> rd((double *)fxs_smem, nt);
-  Ring<float, FXS_NF, FXS_STG> rf((float *)(fxs_smem + Ring<double, FXS_ND, FXS_STG>::bytes(nt)), nt);
-  float *F = e.flx;
-  auto fetch = [&](int s, int64_t g) {
-#pragma unroll
-    for (int p = 0; p < 5; p++) cp_async<8>(rd.at(s, p), e.qa + g + p * N);
-#pragma unroll
-    for (int p = 0; p < 3; p++) {
-      cp_async<4>(rf.at(s, p), e.xim + g + p * N);
-      cp_async<4>(rf.at(s, 3 + p), e.etm + g + p * N);
-      cp_async<4>(rf.at(s, 6 + p), e.zem + g + p * N);
-      cp_async<4>(rf.at(s, 23 + p), e.prim + g + p * N);
-    }
-#pragma unroll
-    for (int p = 0; p < 12; p++) cp_async<4>(rf.at(s, 9 + p), e.dv + g + p * N);
-    cp_async<4>(rf.at(s, 21), e.yaco + g);
-    cp_async<4>(rf.at(s, 22), e.mu + g);
-    cp_async<4>(rf.at(s, 26), e.p + g);
-  };
   TILE_LOOP(e, T) {
     const Scheme &S = e.sc[T.cs];
     const Scalars &SC = e.scal[T.cs];
     const float u1 = (float)SC.umf[1], u2 = (float)SC.umf[2], u3 = (float)SC.umf[3];
-    const ViscConst<float> V(S);
+    const ViscConst<float> C(S);
     const double rhooo = S.rhooo, rhoE_inf = S.hamm1 * S.poo;
     const float poo = (float)S.poo;
-    staged_points<FXS_STG>(T, fetch, [&](int s, int64_t g) {
-      const FluxStageIn in{rf.at(s, 0), rd.at(s, 0), nt};
-      const float x1 = in.at(0), x2 = in.at(1), x3 = in.at(2);
-      const float e1 = in.at(3), e2 = in.at(4), e3 = in.at(5);
-      const float z1 = in.at(6), z2 = in.at(7), z3 = in.at(8);
-      float tv[9];
-      stress_point<float>(in, V, x1, x2, x3, e1, e2, e3, z1, z2, z3, tv);
-      const float pp = in.at(26);
-      // contravariant velocities of u and of umf apart (the freestream split of k_flux)
-      const float r1 = in.vel(0), r2 = in.vel(1), r3 = in.vel(2);
-      const float su1 = x1 * r1 + x2 * r2 + x3 * r3, sm1 = x1 * u1 + x2 * u2 + x3 * u3;
-      const float su2 = e1 * r1 + e2 * r2 + e3 * r3, sm2 = e1 * u1 + e2 * u2 + e3 * u3;
-      const float su3 = z1 * r1 + z2 * r2 + z3 * r3, sm3 = z1 * u1 + z2 * u2 + z3 * u3;
-      const float s1 = su1 + sm1, s2 = su2 + sm2, s3 = su3 + sm3;
-      const double q1 = rd.get(s, 0);
-      const float q = cvt<float>(q1), qp = cvt<float>(q1 - rhooo);
-      F[g] = q * su1 + qp * sm1; F[g + N] = q * su2 + qp * sm2; F[g + 2 * N] = q * su3 + qp * sm3;
-      // the viscous terms are summed before they meet the inviscid flux (small terms first)
-      const float ta[3] = {tv[0], tv[3], tv[5]}, tb[3] = {tv[3], tv[1], tv[4]}, tc[3] = {tv[5], tv[4], tv[2]};
-      const float xm[3] = {x1, x2, x3}, em[3] = {e1, e2, e3}, zm[3] = {z1, z2, z3};
+    GROUP_LOOP(T, g, V) {
+      float f[27][V];
+      double qd[5][V];
 #pragma unroll
-      for (int m = 2; m <= 4; m++) {
-        const float qm = cvt<float>(rd.get(s, m - 1));
-        const float a = qm * s1 + xm[m - 2] * pp - (x1 * ta[m - 2] + x2 * tb[m - 2] + x3 * tc[m - 2]);
-        const float b = qm * s2 + em[m - 2] * pp - (e1 * ta[m - 2] + e2 * tb[m - 2] + e3 * tc[m - 2]);
-        const float c = qm * s3 + zm[m - 2] * pp - (z1 * ta[m - 2] + z2 * tb[m - 2] + z3 * tc[m - 2]);
-        F[g + ((m - 1) * 3 + 0) * N] = a;
-        F[g + ((m - 1) * 3 + 1) * N] = b;
-        F[g + ((m - 1) * 3 + 2) * N] = c;
+      for (int p = 0; p < 5; p++) vload<V, true>(qd[p], e.qa + g + p * N);
+#pragma unroll
+      for (int p = 0; p < 3; p++) {
+        vload<V, true>(f[p], e.xim + g + p * N);
+        vload<V, true>(f[3 + p], e.etm + g + p * N);
+        vload<V, true>(f[6 + p], e.zem + g + p * N);
+        vload<V, true>(f[23 + p], e.prim + g + p * N);
       }
-      // (rhoE + p) U - p (umf . grad xi) - rhoE_inf (umf . grad xi), less the heat-flux terms
-      const double q5 = rd.get(s, 4);
-      const float d5 = cvt<float>(q5) + poo + pp, re = cvt<float>(q5 - rhoE_inf);
-      const float ha = tv[6], hb = tv[7], hc = tv[8];
-      F[g + 12 * N] = d5 * su1 + re * sm1 - (x1 * ha + x2 * hb + x3 * hc);
-      F[g + 13 * N] = d5 * su2 + re * sm2 - (e1 * ha + e2 * hb + e3 * hc);
-      F[g + 14 * N] = d5 * su3 + re * sm3 - (z1 * ha + z2 * hb + z3 * hc);
-    });
+#pragma unroll
+      for (int p = 0; p < 12; p++) vload<V>(f[9 + p], e.dv + g + p * N);
+      vload<V, true>(f[21], e.yaco + g);
+      vload<V, true>(f[22], e.mu + g);
+      vload<V, true>(f[26], e.p + g);
+      float F[15][V];
+#pragma unroll
+      for (int v = 0; v < V; v++) {
+        FluxIn in;
+#pragma unroll
+        for (int p = 0; p < 27; p++) in.f[p] = f[p][v];
+        const double qq[7] = {qd[0][v], qd[1][v], qd[2][v], qd[3][v], qd[4][v], qd[0][v] - rhooo, qd[4][v] - rhoE_inf};
+        narrow_all<7>(qq, in.q);
+        const float x1 = in.at(0), x2 = in.at(1), x3 = in.at(2);
+        const float e1 = in.at(3), e2 = in.at(4), e3 = in.at(5);
+        const float z1 = in.at(6), z2 = in.at(7), z3 = in.at(8);
+        float tv[9];
+        stress_point<float>(in, C, x1, x2, x3, e1, e2, e3, z1, z2, z3, tv);
+        const float pp = in.at(26);
+        // contravariant velocities of u and of umf apart (the freestream split of k_flux)
+        const float r1 = in.vel(0), r2 = in.vel(1), r3 = in.vel(2);
+        const float su1 = x1 * r1 + x2 * r2 + x3 * r3, sm1 = x1 * u1 + x2 * u2 + x3 * u3;
+        const float su2 = e1 * r1 + e2 * r2 + e3 * r3, sm2 = e1 * u1 + e2 * u2 + e3 * u3;
+        const float su3 = z1 * r1 + z2 * r2 + z3 * r3, sm3 = z1 * u1 + z2 * u2 + z3 * u3;
+        const float s1 = su1 + sm1, s2 = su2 + sm2, s3 = su3 + sm3;
+        const float q = in.q[0], qp = in.q[5];
+        F[0][v] = q * su1 + qp * sm1; F[1][v] = q * su2 + qp * sm2; F[2][v] = q * su3 + qp * sm3;
+        // the viscous terms are summed before they meet the inviscid flux (small terms first)
+        const float ta[3] = {tv[0], tv[3], tv[5]}, tb[3] = {tv[3], tv[1], tv[4]}, tc[3] = {tv[5], tv[4], tv[2]};
+        const float xm[3] = {x1, x2, x3}, em[3] = {e1, e2, e3}, zm[3] = {z1, z2, z3};
+#pragma unroll
+        for (int m = 2; m <= 4; m++) {
+          const float qm = in.q[m - 1];
+          F[(m - 1) * 3 + 0][v] = qm * s1 + xm[m - 2] * pp - (x1 * ta[m - 2] + x2 * tb[m - 2] + x3 * tc[m - 2]);
+          F[(m - 1) * 3 + 1][v] = qm * s2 + em[m - 2] * pp - (e1 * ta[m - 2] + e2 * tb[m - 2] + e3 * tc[m - 2]);
+          F[(m - 1) * 3 + 2][v] = qm * s3 + zm[m - 2] * pp - (z1 * ta[m - 2] + z2 * tb[m - 2] + z3 * tc[m - 2]);
+        }
+        // (rhoE + p) U - p (umf . grad xi) - rhoE_inf (umf . grad xi), less the heat-flux terms
+        const float d5 = in.q[4] + poo + pp, re = in.q[6];
+        const float ha = tv[6], hb = tv[7], hc = tv[8];
+        F[12][v] = d5 * su1 + re * sm1 - (x1 * ha + x2 * hb + x3 * hc);
+        F[13][v] = d5 * su2 + re * sm2 - (e1 * ha + e2 * hb + e3 * hc);
+        F[14][v] = d5 * su3 + re * sm3 - (z1 * ha + z2 * hb + z3 * hc);
+      }
+      put_group<V, 15>(e.flx + g, N, T, g, F);
+    }
   }
 }
 
 // divergence de(:,m) = rr1+rr2+rr3 (src/Main3D.f90:722...) plus the sponge of
-// spongego (src/SingleTurbulence3D.f90:368-372) on sponge points
-template <typename R>
-// (the kernel streams: eight CTAs of 256 threads an SM, at most 32 registers a thread)
-__global__ void __launch_bounds__(256, 8) k_div(Eng<R> e) {
+// spongego (src/SingleTurbulence3D.f90:368-372) on sponge points.  The traffic
+// bounds it (mixed 100 B a point without the sponge: 364 us at 24.6 M points;
+// FP64 176 B: 231 us at 8.85 M).  The mixed path takes two points a thread
+// where every plane starts on a pair: 475 -> 420 us (one point: 458); FP64 one
+// point a thread, six CTAs an SM (two points: 280).  The sponge zone is a thin
+// layer and its FP64 work stands behind a real branch (predicated, it was issued
+// for every point): FP64 336 -> 268 us.
+template <typename R, int V>
+__global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_div(const __grid_constant__ Eng<R> e) {
   const int64_t N = e.N;
   TILE_LOOP(e, T) {
     const Scheme &S = e.sc[T.cs];
     Scalars &SC = e.scal[T.cs];
     const R ham = (R)S.ham;
-    const R *F = e.flx;
-    R u1 = 0, u2 = 0, u3 = 0;
+    R u1 = 0, u2 = 0, u3 = 0, r0 = 0, p0 = 0, e0 = 0;
     if constexpr (Freestream<R>::on) {
       u1 = (R)SC.umf[1]; u2 = (R)SC.umf[2]; u3 = (R)SC.umf[3];
+      r0 = (R)S.rhooo; p0 = (R)S.poo; e0 = (R)(S.hamm1 * S.poo);
     }
-    POINT_LOOP(T, g) {
-      const R as = e.asz[g], bs = e.bsz[g];
-      const bool sponge = as != (R)0 || bs != (R)0;
-      // the mixed path: the sponge zone is a thin layer, and warps without a sponge point skip its FP64
-      // subtractions and conversions (a warp vote makes the branch a real one; a per-point test was
-      // predicated and issued that FP64 work everywhere).  The FP64 kernel streams and keeps one variant.
-      const bool any_sponge = Freestream<R>::on ? __any_sync(__activemask(), sponge) : true;
-      R fs[5] = {0, 0, 0, 0, 0};
+    GROUP_LOOP(T, g, V) {
+      R F[15][V], as[V], bs[V], d[5][V];
+      vload<V>(as, e.asz + g);
+      vload<V>(bs, e.bsz + g);
+#pragma unroll
+      for (int c = 0; c < 15; c++) vload<V>(F[c], e.flx + g + c * N);
+      R gm[3][V];
       if constexpr (Freestream<R>::on) {
-        // divergence of the freestream fluxes: rho_inf, p_inf, rhoE_inf times the metric divergence
-        const R g1 = e.gm[g], g2 = e.gm[g + N], g3 = e.gm[g + 2 * N];
-        const R ug = u1 * g1 + u2 * g2 + u3 * g3;
-        fs[0] = (R)S.rhooo * ug;
-        fs[1] = (R)S.poo * g1; fs[2] = (R)S.poo * g2; fs[3] = (R)S.poo * g3;
-        fs[4] = (R)(S.hamm1 * S.poo) * ug;
+#pragma unroll
+        for (int c = 0; c < 3; c++) vload<V>(gm[c], e.gm + g + c * N);
       }
-      // two versions of the point's update, chosen per warp
-      auto update = [&](auto with_sponge) {
-  #pragma unroll
-        for (int m = 1; m <= 5; m++) {
-          R d = F[g + ((m - 1) * 3 + 0) * N] + F[g + ((m - 1) * 3 + 1) * N] + F[g + ((m - 1) * 3 + 2) * N];
-          if constexpr (Freestream<R>::on) d = d + fs[m - 1];
-          if (decltype(with_sponge)::value && sponge) {
-            if constexpr (Freestream<R>::on) {  // the pressure plane already holds p - p_inf, p_inf = 1/gamma
-              if (m == 1) d = d + as * cvt<R>(e.qa[g] - 1.0);
-              else if (m <= 4) d = d + as * cvt<R>(e.qa[g + (m - 1) * N]);
-              else d = d + bs * e.p[g];
-            } else {
-              if (m == 1) d = d + as * (cvt<R>(e.qa[g]) - (R)1);
-              else if (m <= 4) d = d + as * (cvt<R>(e.qa[g + (m - 1) * N]) - (R)0);
-              else d = d + bs * (e.p[g] - ham * (R)1);
-            }
-          }
-          e.de[g + (m - 1) * N] = d;
+      bool sponge = false;
+#pragma unroll
+      for (int v = 0; v < V; v++) {
+        sponge |= as[v] != (R)0 || bs[v] != (R)0;
+#pragma unroll
+        for (int m = 0; m < 5; m++) d[m][v] = F[m * 3][v] + F[m * 3 + 1][v] + F[m * 3 + 2][v];
+        if constexpr (Freestream<R>::on) {
+          // divergence of the freestream fluxes: rho_inf, p_inf, rhoE_inf times the metric divergence
+          const R ug = u1 * gm[0][v] + u2 * gm[1][v] + u3 * gm[2][v];
+          d[0][v] = d[0][v] + r0 * ug;
+#pragma unroll
+          for (int m = 1; m < 4; m++) d[m][v] = d[m][v] + p0 * gm[m - 1][v];
+          d[4][v] = d[4][v] + e0 * ug;
         }
-      };
-      if (!Freestream<R>::on || any_sponge) update(std::true_type{});
-      else update(std::false_type{});
+      }
+      if (sponge) {
+        keep_branch();
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+          if (as[v] == (R)0 && bs[v] == (R)0) continue;
+          const int64_t q = g + v;
+          if constexpr (Freestream<R>::on) {  // the pressure plane already holds p - p_inf, p_inf = 1/gamma
+            const double qd[4] = {e.qa[q] - 1.0, e.qa[q + N], e.qa[q + 2 * N], e.qa[q + 3 * N]};
+            float qf[4];
+            narrow_all<4>(qd, qf);
+#pragma unroll
+            for (int m = 0; m < 4; m++) d[m][v] = d[m][v] + as[v] * qf[m];
+            d[4][v] = d[4][v] + bs[v] * e.p[q];
+          } else {
+            d[0][v] = d[0][v] + as[v] * (cvt<R>(e.qa[q]) - (R)1);
+#pragma unroll
+            for (int m = 1; m < 4; m++) d[m][v] = d[m][v] + as[v] * (cvt<R>(e.qa[q + m * N]) - (R)0);
+            d[4][v] = d[4][v] + bs[v] * (e.p[q] - ham * (R)1);
+          }
+        }
+      }
+      put_group<V, 5>(e.de + g, N, T, g, d);
     }
   }
 }
@@ -3234,8 +3305,6 @@ static cudaError_t seg_attr() {
 cudaError_t seg_init() {
   cudaError_t e = seg_attr<float, float>();
   if (e == cudaSuccess) e = seg_attr<double, double>();
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_flux_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flux_staged_smem(256));
   return e;
 }
 
@@ -3304,10 +3373,18 @@ static void pointwise_t(const Eng<R> &eng, cudaStream_t st, int which) {
         k_flux<R><<<g, t, 0, st>>>(e);
         break;
       }
-      if constexpr (Freestream<R>::on) k_flux_staged<<<g, t, flux_staged_smem(t), st>>>(e);
+      if constexpr (Freestream<R>::on) {
+        if (e.N % 2 == 0) k_flux_mixed<2><<<g, t, 0, st>>>(e);
+        else k_flux_mixed<1><<<g, t, 0, st>>>(e);
+      }
       break;
-    case PW_DIV: k_div<R><<<g, t, 0, st>>>(e); break;
-    case PW_RK: k_rk<R><<<g, t, 0, st>>>(e); break;
+    case PW_DIV:
+      if (Freestream<R>::on && e.N % 2 == 0) k_div<R, 2><<<g, t, 0, st>>>(e);
+      else k_div<R, 1><<<g, t, 0, st>>>(e);
+      break;
+    case PW_RK:
+      k_rk<R><<<g, t, 0, st>>>(e);
+      break;
   }
 }
 void pointwise_d(const Eng<double> &e, cudaStream_t st, int which) { pointwise_t<double>(e, st, which); }
