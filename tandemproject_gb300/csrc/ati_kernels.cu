@@ -2923,6 +2923,7 @@ __device__ void scalar_op(const Scheme &S, Scalars &s, int op, int nk) {
     const double dtko = s.dt * min(max(nk - 2, 0), 1) / (nkrk - nk + 3);
     const double dtk = s.dt * min(nk - 1, 1) / (nkrk - nk + 2);
     d_movef(S, s, dtko, dtk);
+    if (nk > 1) s.dtk = s.dt / (nkrk - nk + 1);
   } else if (op == SC_CFL_RESET) {
     s.cflmax[0] = 0ull; s.cflmax[1] = 0ull;
   } else if (op == SC_DT_NEW) {  // n % 10 == 1: new dt target
@@ -2940,11 +2941,11 @@ __device__ void scalar_op(const Scheme &S, Scalars &s, int op, int nk) {
   } else if (op == SC_DT) {
     const double sn = sin(0.05 * S.pi * (double)(s.n - s.ndt));
     s.dt = s.dts + (s.dte - s.dts) * (sn * sn);
+    s.dtk = s.dt / (nkrk - nk + 1);  // (the first stage's; SC_MOVEF_A takes the later ones')
   } else if (op == SC_MOVEF_B) {
     const double dtko = s.dt * min(nk - 1, 1) / (nkrk - nk + 2);
     const double dtk = s.dt / (nkrk - nk + 1);
-    d_movef(S, s, dtko, dtk);
-    s.dtk = dtk;
+    d_movef(S, s, dtko, dtk);  // (the RK update may run beside this: its factor s.dtk is set already)
   } else if (op == SC_ADVANCE) {
     s.n = s.n + 1;
     s.timo = s.timo + s.dt;
