@@ -46,6 +46,8 @@ thread_local std::string g_tma_err;  // a tensor-map encoding failure at creatio
 
 }  // namespace
 
+constexpr int NSIDE = 6;  // side streams: two directions and some classes of line lengths at once
+
 struct ati_handle {
   ati_config_t cfg{};  // case 0; the numerics every case of a batch shares
   int nb = 0;
@@ -88,9 +90,9 @@ struct ati_handle {
   int maxlen[4] = {0, 0, 0, 0};
   int maxlines[4] = {0, 0, 0, 0};
   cudaStream_t st = nullptr;
-  // side streams and events for the three directions' sweeps, which are independent within a stage
-  cudaStream_t side[2] = {nullptr, nullptr};
-  cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
+  // side streams and events for a stage's independent sweeps (directions, classes of line lengths)
+  cudaStream_t side[NSIDE] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[NSIDE] = {};
   // and for the scalars of a stage (one thread a case, FP64 sines), beside the kernels that do not read them
   cudaStream_t scal_st = nullptr;
   cudaEvent_t ev_scal[2] = {nullptr, nullptr};
@@ -1447,9 +1449,9 @@ static int create_impl(const ati_config_t *cfgs, int ncase, ati_handle_t **out) 
     dzm32.assign(dzm.begin(), dzm.end());
   }
   e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
-  for (int q = 0; q < 2 && e == cudaSuccess; q++) e = cudaStreamCreateWithFlags(&h->side[q], cudaStreamNonBlocking);
+  for (int q = 0; q < NSIDE && e == cudaSuccess; q++) e = cudaStreamCreateWithFlags(&h->side[q], cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
-  for (int q = 0; q < 2 && e == cudaSuccess; q++) e = cudaEventCreateWithFlags(&h->ev_join[q], cudaEventDisableTiming);
+  for (int q = 0; q < NSIDE && e == cudaSuccess; q++) e = cudaEventCreateWithFlags(&h->ev_join[q], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->scal_st, cudaStreamNonBlocking);
   for (int q = 0; q < 2 && e == cudaSuccess; q++) e = cudaEventCreateWithFlags(&h->ev_scal[q], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->arena, 0, bytes, h->st);
@@ -1582,7 +1584,7 @@ extern "C" int ati_destroy(ati_handle_t *h) {
     if (p) cudaFree(p);
   if (h->arena) cudaFree(h->arena);
   if (h->st) cudaStreamDestroy(h->st);
-  for (int q = 0; q < 2; q++) {
+  for (int q = 0; q < NSIDE; q++) {
     if (h->side[q]) cudaStreamDestroy(h->side[q]);
     if (h->ev_join[q]) cudaEventDestroy(h->ev_join[q]);
   }
@@ -2282,23 +2284,46 @@ static int autotune_t(ati_handle *h, Eng<R> &e) {
 
 static int autotune(ati_handle *h) { return h->mixed ? autotune_t<float>(h, h->ef) : autotune_t<double>(h, h->ed); }
 
-// The derivative sweeps of the three directions within a stage read and write
-// disjoint planes and face buffers, so xi runs on the handle's stream and eta,
-// zeta on two side streams forked from and joined back into it (inside the step
-// graph too): each direction alone leaves the GPU under-occupied.  With
-// profiling on they run one after another, so each launch is timed alone.
-template <typename F>
-static void three_directions(ati_handle *h, F &&sweep) {
-  if (h->profiling) {
-    for (int nn = 3; nn >= 1; nn--) sweep(nn, h->st);
+// The derivative sweeps of the three directions within a stage read and write disjoint planes and face buffers, and so
+// do a direction's classes (lines of equal segment counts, one launch each): the first runs on the handle's stream and
+// the others on side streams forked from and joined back into it (inside the step graph too).  Each alone leaves the
+// GPU under-occupied, and one after another every class would end in a tail of its own.  Step of 0.23 M points in FP64
+// (xi lines of 49 and 121 points) 1331 -> 967 us, of 0.61 M points 2769 -> 2655 us, five mixed cases of 17 M points
+// 14.81 -> 14.53 ms.  With profiling on they run one after another, so each launch is timed alone.
+template <typename R>
+static int sweep_parts(const Eng<R> &e, bool strict, int nn, bool filt) {
+  if (std::is_same<R, double>::value && (strict || !e.fx_ok[filt][nn])) return 1;
+  if (std::is_same<R, float>::value && nn == 3 && !filt && e.dense && e.dzl > 0) return 1;
+  return std::max(1, e.nsegc[nn]);
+}
+// the engine with class c alone in direction nn (lines outside the classes go with the first one)
+template <typename R>
+static Eng<R> sweep_part(const Eng<R> &e, int nn, int c) {
+  Eng<R> p = e;
+  p.nsegc[nn] = 1;
+  p.segc[nn][0] = e.segc[nn][c];
+  if (c > 0) p.nlt_fx[nn] = p.nlt[nn];
+  return p;
+}
+// sweep(nn, stream, engine) over the directions n1..n2 and their classes at once
+template <typename R, typename F>
+static void sweep_all(ati_handle *h, const Eng<R> &e, int n1, int n2, bool filt, F &&sweep) {
+  const bool strict = h->cfg.precision == ATI_FP64_STRICT;
+  int np = 0;
+  for (int nn = n1; nn <= n2; nn++) np += sweep_parts(e, strict, nn, filt);
+  if (h->profiling || np == 1) {
+    for (int nn = n2; nn >= n1; nn--) sweep(nn, h->st, e);
     return;
   }
   cudaEventRecord(h->ev_fork, h->st);
-  for (int q = 0; q < 2; q++) cudaStreamWaitEvent(h->side[q], h->ev_fork, 0);
-  sweep(1, h->st);
-  sweep(2, h->side[0]);
-  sweep(3, h->side[1]);
-  for (int q = 0; q < 2; q++) {
+  const int ns = std::min(np - 1, NSIDE);
+  for (int q = 0; q < ns; q++) cudaStreamWaitEvent(h->side[q], h->ev_fork, 0);
+  int q = 0;
+  for (int nn = n1; nn <= n2; nn++) {
+    const int n = sweep_parts(e, strict, nn, filt);
+    for (int c = 0; c < n; c++, q++) sweep(nn, q == 0 ? h->st : h->side[(q - 1) % ns], n > 1 ? sweep_part(e, nn, c) : e);
+  }
+  for (q = 0; q < ns; q++) {
     cudaEventRecord(h->ev_join[q], h->side[q]);
     cudaStreamWaitEvent(h->st, h->ev_join[q], 0);
   }
@@ -2319,7 +2344,9 @@ static int filter_step_t(ati_handle *h, const Eng<R> &e) {
   for (int nn = 1; nn <= 3; nn++) {
     SweepIO<double, double> io{h->ed.qa, N, h->ed.qa, N, nn == 3 ? h->ed.qo : nullptr, 5, 1, false};
     for (int f = 0; f < 5; f++) io.ofs[f] = fo.v[f];
-    PROF(h, ATI_K_FILTER_XI + nn - 1, C::qsweep(strict, e, h->st, nn, io));
+    sweep_all(h, e, nn, nn, true, [&](int nn, cudaStream_t s, const Eng<R> &e) {
+      PROF(h, ATI_K_FILTER_XI + nn - 1, C::qsweep(strict, e, s, nn, io));
+    });
   }
   CKL();
   return ATI_OK;
@@ -2344,7 +2371,7 @@ static int rk_stage_t(ati_handle *h, const Eng<R> &e, int nk, bool keep_recv) {
   // The stage's scalars are one thread a case, some microseconds of FP64 sines and cosines: they run on a stream of
   // their own beside the primitives and the gradients (the frame's velocity, first read by the CFL maxima and the
   // fluxes; the time step) and beside the RK update (the frame at the stage's end), whose factor the earlier ones
-  // set.  With profiling on they run one after another, like the three directions.
+  // set.  With profiling on they run one after another, like the sweeps.
   // (a step of 0.23 M points in FP64 1357 -> 1320 us, of 0.86 M points in the mixed path 1115 -> 1047 us)
   const cudaStream_t ss = h->profiling ? st : h->scal_st;
   auto fork = [&] {
@@ -2380,7 +2407,7 @@ static int rk_stage_t(ati_handle *h, const Eng<R> &e, int nk, bool keep_recv) {
     // d(u,v,w,T)/d(zeta,eta,xi) (src/Main3D.f90:629-651): four fields per launch
     PROF(h, ATI_K_MPIGO, C::mpigo(strict, e, st, tp(h, mpt), mpt.n, mpt.maxline, 0, e.prim,
                                   e.prim, e.prim, N, 4));
-    three_directions(h, [&](int nn, cudaStream_t s) {
+    sweep_all(h, e, 1, 3, false, [&](int nn, cudaStream_t s, const Eng<R> &e) {
       SweepIO<R, R> io{e.prim, N, e.dv + (nn - 1) * N, 3 * N, nullptr, 4, 2, true};
       PROF(h, ATI_K_DERIV_XI + nn - 1, C::sweep(strict, e, s, nn, false, io));
     });
@@ -2397,7 +2424,7 @@ static int rk_stage_t(ati_handle *h, const Eng<R> &e, int nk, bool keep_recv) {
   if (own && !Freestream<R>::on && keep_recv)
     PROF(h, ATI_K_MPIGO, C::mpigo(strict, e, st, tp(h, h->tl_mpigo), h->tl_mpigo.n, h->tl_mpigo.maxline, 0, e.flx,
                                   e.flx + N, e.flx + 2 * N, 3 * N, 1));
-  three_directions(h, [&](int nn, cudaStream_t s) {
+  sweep_all(h, e, 1, 3, false, [&](int nn, cudaStream_t s, const Eng<R> &e) {
     SweepIO<R, R> io{e.flx + (nn - 1) * N, 3 * N, e.flx + (nn - 1) * N, 3 * N, nullptr, 5, 1, true};
     PROF(h, ATI_K_DERIV_XI + nn - 1, C::sweep(strict, e, s, nn, false, io));
   });
