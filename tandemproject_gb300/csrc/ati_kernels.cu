@@ -2063,6 +2063,25 @@ struct PlaneIn {
   __device__ R vel(int k) const { return e.prim[g + k * N]; }
 };
 
+// (-1/J)^1.5 of the LES term, J < 0, and the root of the strain invariant.  The fast build takes them from the refined
+// approximations (recip_nr, rsqrt_nr: a few ulp, as pow) in some twenty FP64 operations; pow and sqrt took half of the
+// stress kernel's two hundred, which the FP64 pipe bounds (a step with the LES term of 0.61 M points 2669 -> 2340 us).
+__device__ __forceinline__ double volume_15(double yac) {
+  if constexpr (kFast) {
+    const double t = recip_nr(-yac);
+    return t * (t * rsqrt_nr(t));
+  }
+  return pow(-1.0 / yac, 1.5);
+}
+__device__ __forceinline__ float root(float x) { return sqrt(x); }
+__device__ __forceinline__ double root(double x) {
+  if constexpr (kFast) {
+    if (x > 1e-280 && x < 1e280) return x * rsqrt_nr(x);
+    keep_branch();  // zero (a uniform state) and what the approximation does not cover
+  }
+  return sqrt(x);
+}
+
 // physical gradients of u, v, w, T and the viscous stresses and heat fluxes at one point
 // (src/Main3D.f90:631-692), from the twelve derivative planes dv and the point's metrics:
 // t = txx, tyy, tzz, txy, tyz, tzx and the energy terms hxx, hyy, hzz.  In gives the point's
@@ -2088,9 +2107,9 @@ __device__ __forceinline__ void stress_point(const In &in, const ViscConst<R> &V
   if (V.les == 1) {
     const R d1 = txx * txx + tyy * tyy + tzz * tzz + (hzz + txy) * (hzz + txy) + (hyy + tzx) * (hyy + tzx) +
                  (hxx + tyz) * (hxx + tyz);
-    const R varr = (R)pow(-1.0 / (double)yac, 1.5);
+    const R varr = (R)volume_15(yac);
     const R q1 = in.rho();
-    r3 = q1 * (V.sm1 * V.sm1) * varr * sqrt((R)2 * d1);
+    r3 = q1 * (V.sm1 * V.sm1) * varr * root((R)2 * d1);
     r1 = r1 + r3 * yac;
     r2 = r2 + V.tgp * r3 * yac;
     r3 = V.tt * (q1 * V.sm2 * varr * d1);
