@@ -295,7 +295,9 @@ int ati_launch_count(ati_handle_t *h, int64_t *count);
  * out[2] zeta lines per CTA, out[3] points per tile of the flux kernel.
  * ati_init picks out[1..2] and, per pointwise kernel, the points per tile by
  * timing candidates on the handle's own grid (results do not depend on them:
- * every line and point is computed the same way). */
+ * every line and point is computed the same way; the segmented sweeps of the
+ * mixed path and of the FP64 fast path have tiles of a fixed shape, and
+ * out[1..2] concern the lines those do not take). */
 int ati_tiles(ati_handle_t *h, int32_t out[4]);
 /* Pins the tile shapes (same meaning as ati_tiles; 0 keeps the current value;
  * in[3] then applies to every pointwise kernel): in[0] must be 0 or the fixed

@@ -2064,19 +2064,25 @@ struct PlaneIn {
 };
 
 // (-1/J)^1.5 of the LES term, J < 0, and the root of the strain invariant.  The fast build takes them from the refined
-// approximations (recip_nr, rsqrt_nr: a few ulp, as pow) in some twenty FP64 operations; pow and sqrt took half of the
-// stress kernel's two hundred, which the FP64 pipe bounds (a step with the LES term of 0.61 M points 2669 -> 2340 us).
+// approximations (recip_nr, rsqrt_nr) and one correction of the root by its residual, some twenty-five FP64 operations;
+// pow and sqrt took half of the stress kernel's two hundred, which the FP64 pipe bounds (a step with the LES term of
+// 0.61 M points 2669 -> 2358 us).  Largest errors measured over 2^-60 .. 2^60, in units of the last place: the power
+// 2.26 (with pow 2.28), the root 0.50 (sqrt 0.50).
+__device__ __forceinline__ double root_nr(double x) {
+  const double y = rsqrt_nr(x), s = x * y;
+  return fma(0.5 * y, fma(-s, s, x), s);
+}
 __device__ __forceinline__ double volume_15(double yac) {
   if constexpr (kFast) {
     const double t = recip_nr(-yac);
-    return t * (t * rsqrt_nr(t));
+    return t * root_nr(t);
   }
   return pow(-1.0 / yac, 1.5);
 }
 __device__ __forceinline__ float root(float x) { return sqrt(x); }
 __device__ __forceinline__ double root(double x) {
   if constexpr (kFast) {
-    if (x > 1e-280 && x < 1e280) return x * rsqrt_nr(x);
+    if (x > 1e-280 && x < 1e280) return root_nr(x);
     keep_branch();  // zero (a uniform state) and what the approximation does not cover
   }
   return sqrt(x);
