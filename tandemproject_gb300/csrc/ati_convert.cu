@@ -51,8 +51,7 @@ __global__ void k_check_conv(int64_t n, unsigned long long *bad) {
       default: break;
     }
     const double d = __longlong_as_double((long long)db);
-    const float na = ati::narrow(d), nb2 = (float)d;
-    if (!((na != na && nb2 != nb2) || __float_as_uint(na) == __float_as_uint(nb2))) nb++;
+    const float nb2 = (float)d;
     float nv[1];
     ati::narrow_all<1>({d}, nv);
     if (!((nv[0] != nv[0] && nb2 != nb2) || __float_as_uint(nv[0]) == __float_as_uint(nb2))) nb++;

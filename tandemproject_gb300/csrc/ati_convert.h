@@ -1,4 +1,4 @@
-// ati_convert.h — FP32 -> FP64 conversion on the integer pipes.
+// ati_convert.h — conversions between FP32 and FP64 on the integer pipes.
 //
 // On GB300 the FP64 pipe does 1/55 of the FP32 work per clock and also executes
 // the F2F conversion instructions, so the mixed path's RK update and filter,
@@ -22,24 +22,6 @@ __device__ __forceinline__ double widen(float f) {
   if (e - 1u < 254u) return __hiloint2double((int)(s | ((e + 896u) << 20) | (m >> 3)), (int)(m << 29));
   if ((u << 1) == 0u) return __hiloint2double((int)s, 0);  // signed zero
   return (double)f;  // subnormal, infinity, NaN
-}
-
-// double -> float, rounded to nearest even, for results in the normal float range:
-// the significand's top 23 bits plus a rounding increment decided by the 29 bits
-// dropped (above half, or exactly half with an odd result); a carry out of the
-// significand moves into the exponent, as the rounding requires (up to infinity).
-// Zero, results below the normal range, overflow, infinities and NaNs fall back
-// to the instruction.  Bit for bit the instruction's result (checked on the device
-// by ati_check_conversions).
-__device__ __forceinline__ float narrow(double d) {
-  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
-  const unsigned e = (hi >> 20) & 0x7ffu;
-  if (e - 897u < 254u) {  // float exponent e - 896 in 1..254
-    const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29), r = lo & 0x1fffffffu;
-    const unsigned f = (hi & 0x80000000u) | ((e - 896u) << 23) | m;
-    return __uint_as_float(f + (unsigned)((r > 0x10000000u) | ((r == 0x10000000u) & (m & 1u))));
-  }
-  return (float)d;
 }
 
 // 1/a and 1/sqrt(a) for the FP64 fast build, for positive normal a: the
@@ -77,6 +59,8 @@ __device__ __forceinline__ void keep_branch() { asm volatile("nanosleep.u32 0;")
 // predicates the conversion instruction, and a predicated-off F2F still takes its turn in the FP64 pipe: the mixed
 // filter sweeps spent 3.8 FP64 instructions a point and field, 1.4 of them its own additions.  Results are the
 // instruction's, bit for bit (checked on the device by ati_check_conversions).
+// Narrowing rounds to nearest even: the significand's top 23 bits and a carry decided by the 29 bits dropped, which may
+// run into the exponent, as the rounding requires (up to infinity).
 template <int K>
 __device__ __forceinline__ void narrow_all(const double (&v)[K], float (&o)[K]) {
   bool odd = false;
@@ -110,12 +94,8 @@ __device__ __forceinline__ void widen_all(const float (&v)[K], double (&o)[K]) {
   }
 }
 
-// conversion between the engine types: FP32 -> FP64 on the integer pipes.  The
-// other direction stays with the conversion instruction here: rounding takes some
-// 15 integer operations and branches, slower in the line sweeps' load loops than
-// the FP64 pipe it would spare (measured on the mixed filter sweeps), and in the
-// register-bounded flux kernel (297 -> 346 us); the primitives kernel, bound by
-// the FP64 pipe, calls narrow() itself (142 -> 133 us)
+// conversion between the engine types: FP32 -> FP64 on the integer pipes; the other direction is the conversion
+// instruction here, and the kernels whose time it was (filters, fluxes, divergence, primitives) call narrow_all
 template <typename TO, typename TI>
 __device__ __forceinline__ TO cvt(TI v) {
   if constexpr (std::is_same<TO, TI>::value) return v;

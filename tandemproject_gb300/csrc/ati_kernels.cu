@@ -1822,7 +1822,8 @@ __device__ __forceinline__ void put_group(T *o, int64_t N, const PTile &t, int64
 }
 
 // ---------------------------------------------------------------------------
-// Shared-memory staging of the mixed path's streaming kernels.  Each thread
+// Shared-memory staging of the mixed path's primitives (five planes in: with more, plain wide loads are faster, as
+// the groups of points above; unstaged they take 255 us at 24.6 M points, staged 240).  Each thread
 // copies (cp.async) the input planes of the points it will take STG - 1 points
 // ahead into its own column of a ring of STG slots, and waits only for its own
 // oldest copies: the loads of the next points are in flight while it computes,
@@ -1874,28 +1875,31 @@ __device__ __forceinline__ bool prim_point(const Eng<R> &e, const PrimConst<R> &
                                            const double q[5]) {
   const R gamm1 = C.gamm1, gam = C.gam, srefp1dre = C.srefp1dre, srefoo = C.srefoo;
   const double rhoE_inf = C.rhoE_inf;
-  // (the mixed kernel is bound by the FP64 pipe, which also runs the conversion instruction: the state is
-  // rounded to FP32 on the integer pipes instead, bit for bit the same)
-  auto rnd = [](double v) -> R {
-    if constexpr (Freestream<R>::on) return narrow(v);
-    else return (R)v;
-  };
-  // (the FP64 fast build takes its reciprocals and square root from recip_nr / rsqrt_nr: the kernel is bound
-  // by the FP64 pipe, and the IEEE division and square root are its largest users)
+  R qr[5];  // rho, rho u, rho v, rho w, and rho E (mixed: rho E - rho E_inf, taken in FP64 before rounding)
+  if constexpr (Freestream<R>::on) {
+    const double qd[5] = {q[0], q[1], q[2], q[3], q[4] - rhoE_inf};
+    narrow_all<5>(qd, qr);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 5; k++) qr[k] = q[k];
+  }
+  // (the FP64 fast build takes its reciprocals and square root from recip_nr / rsqrt_nr; the mixed path rounds the state
+  // to FP32 on the integer pipes, 245 -> 240 us at 24.6 M points and 18.7 -> 15.3 at 0.9 M against the conversions one
+  // by one)
   constexpr bool NR = kFast && !Freestream<R>::on;
-  const R q1 = rnd(q[0]), q2 = rnd(q[1]), q3 = rnd(q[2]), q4 = rnd(q[3]);
+  const R q1 = qr[0], q2 = qr[1], q3 = qr[2], q4 = qr[3];
   R d1;
   if constexpr (NR) d1 = recip_nr(q1);
   else d1 = (R)1 / q1;
   const R d2 = q2 * d1, d3 = q3 * d1, d4 = q4 * d1;
   R pp, d5;
   if constexpr (Freestream<R>::on) {
-    // p - p_inf from rhoE - rhoE_inf (taken in FP64 before rounding); (gamma-1) rhoE_inf = p_inf
-    const R re = rnd(q[4] - rhoE_inf);
+    // p - p_inf from rhoE - rhoE_inf; (gamma-1) rhoE_inf = p_inf
+    const R re = qr[4];
     pp = gamm1 * (re - (R)0.5 * (q2 * d2 + q3 * d3 + q4 * d4));
     d5 = gam * (C.poo + pp) * d1;
   } else {
-    const R q5 = cvt<R>(q[4]);
+    const R q5 = qr[4];
     pp = gamm1 * (q5 - (R)0.5 * (q2 * d2 + q3 * d3 + q4 * d4));
     d5 = gam * pp * d1;
   }
