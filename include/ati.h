@@ -409,7 +409,7 @@ int ati_check_recip(int64_t n, double worst[2]);
  * stream).
  *  - Allocates and frees nothing.  Its scratch (LU factors; the
  *    forward-elimination values stay in shared memory) is one static device
- *    array of 5*ATI_NOALLOC_MAX_LEN doubles (160 KB) per GPU, held until the
+ *    array of 5*ATI_NOALLOC_MAX_LEN + 1 doubles (160 KB) per GPU, held until the
  *    process exits.
  *  - The first call on each device (and again after a device reset, which
  *    gives the context a new array) looks up the array's device address with
@@ -426,8 +426,10 @@ int ati_check_recip(int64_t n, double worst[2]);
  *    earlier work with ATI_ECUDA (that error is left pending).
  *  - All calls share the one scratch array and it keeps the previous call's
  *    contents: the LU factors depend only on len and are refactored when len
- *    differs from the previous call's, and every other value a call reads it
- *    wrote itself, so nothing needs clearing.  Calls must therefore be
+ *    differs from the previous call's (a captured call's graph looks on the
+ *    device, at each replay, and so does every call after a first captured
+ *    one), and every other value a call reads it wrote itself, so nothing
+ *    needs clearing.  Calls, replays among them, must therefore be
  *    ordered on the GPU: calls that overlap (different streams, no ordering
  *    between them) race on the array and must not be issued. */
 #define ATI_NOALLOC_MAX_POINTS 2000000

@@ -36,9 +36,10 @@ namespace {
 
 constexpr int64_t kMaxPoints = ATI_NOALLOC_MAX_POINTS;
 constexpr int kMaxLen = ATI_NOALLOC_MAX_LEN;
-constexpr int64_t kScratchDoubles = 5 * (int64_t)kMaxLen;
+constexpr int64_t kTag = 5 * (int64_t)kMaxLen;
+constexpr int64_t kScratchDoubles = kTag + 1;
 
-// factor table (5 per line position)
+// factor table (5 per line position), then the line length whose factors it holds
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
 constexpr double kAlpha = 0.5862704032801503, kBeta = 0.09549533555017055;
@@ -51,8 +52,11 @@ struct Rows {
 
 // LU factors of the pentadiagonal left-hand side with one-sided boundary rows
 // at both ends, one thread (the recurrence of penta is sequential).
+// A table that holds this length's factors already is left alone: what it holds is known on the device alone
+// once calls are replayed from graphs.
 __global__ void k_noalloc_factors(double *fac, int len, Rows R) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  if (blockIdx.x != 0 || threadIdx.x != 0 || fac[kTag] == (double)len) return;
+  fac[kTag] = (double)len;
   const int is = 0, ie = len - 1;
   double *f = fac;
   for (int i = 0; i < len; i++)
@@ -190,11 +194,12 @@ int lines_per_cta(int64_t nlines, int len, int nsm) {
 
 std::mutex g_mu;
 // per device: the scratch array's device address, the context it was looked up in, and the line length whose
-// LU factors the array holds (-1: none)
+// LU factors the array holds (-1: unknown; the device's own tag says)
 void *g_ptr[64] = {nullptr};
 void *g_ctx[64] = {nullptr};
 int g_len[64];
 int g_nsm[64];
+bool g_captured[64];  // a call was captured on the device: a replay, unseen here, may change the factors
 bool g_len_init = false;
 
 // cuCtxGetCurrent from the driver, fetched through the runtime (no link-time dependency on libcuda): a device
@@ -267,6 +272,13 @@ extern "C" int ati_deriv_lines_noalloc(const double *in, double *out, int64_t nl
                                       "(not cleared, nothing launched): ") + cudaGetErrorString(pe)).c_str());
     return ATI_ECUDA;
   }
+  cudaStream_t st = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaError_t e = cudaStreamIsCapturing(st, &cap); e != cudaSuccess) {
+    cudaGetLastError();
+    ati_set_thread_error((std::string("ati_deriv_lines_noalloc: ") + cudaGetErrorString(e)).c_str());
+    return ATI_ECUDA;
+  }
   void *base = nullptr;
   bool refactor = false;
   int nsm = 1;
@@ -290,27 +302,31 @@ extern "C" int ati_deriv_lines_noalloc(const double *in, double *out, int64_t nl
       // (a context's kernels have their own attributes: set with the look-up)
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_noalloc_deriv, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)kTileMax);
-      int nsm = 0;
       if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) {
         ati_set_thread_error((std::string("ati_deriv_lines_noalloc: ") + cudaGetErrorString(e)).c_str());
         return ATI_ECUDA;
       }
       g_nsm[dev] = nsm > 0 ? nsm : 1;
-      if (p != g_ptr[dev]) g_len[dev] = -1;  // a new array: no factors yet
+      g_len[dev] = -1;  // a new context's array, at whatever address: no factors yet
       g_ptr[dev] = p;
       g_ctx[dev] = current_ctx();
     }
     base = g_ptr[dev];
     nsm = g_nsm[dev];
-    refactor = g_len[dev] != len;
-    g_len[dev] = len;
+    if (cap != cudaStreamCaptureStatusNone) {
+      // captured, not run: the graph brings its own factor kernel, and from now on so does every call
+      g_captured[dev] = true;
+      refactor = true;
+    } else {
+      refactor = g_captured[dev] || g_len[dev] != len;
+      g_len[dev] = len;
+    }
   }
   double *fac = (double *)base;
-  cudaStream_t st = (cudaStream_t)stream;
   const Rows R = make_rows();
   // the LU factors depend on the line length only: refactored when it changes (calls are ordered on the GPU, so
-  // a call finds the factors of the previous call in the array)
+  // a call finds the factors of the previous call in the array); where calls are captured the kernel itself looks
   if (refactor) k_noalloc_factors<<<1, 1, 0, st>>>(fac, len, R);
   const int lpc = lines_per_cta(nlines, len, nsm);
   const size_t smem = (size_t)lpc * (len | 1) * sizeof(double);
