@@ -2503,11 +2503,12 @@ __global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_div(const __grid_consta
         for (int m = 0; m < 5; m++) d[m][v] = F[m * 3][v] + F[m * 3 + 1][v] + F[m * 3 + 2][v];
         if constexpr (Freestream<R>::on) {
           // divergence of the freestream fluxes: rho_inf, p_inf, rhoE_inf times the metric divergence
+          // (each product rounded before it is added: contracted, the last place of a result in some 10^8 differs)
           const R ug = u1 * gm[0][v] + u2 * gm[1][v] + u3 * gm[2][v];
-          d[0][v] = d[0][v] + r0 * ug;
+          d[0][v] = d[0][v] + __fmul_rn(r0, ug);
 #pragma unroll
-          for (int m = 1; m < 4; m++) d[m][v] = d[m][v] + p0 * gm[m - 1][v];
-          d[4][v] = d[4][v] + e0 * ug;
+          for (int m = 1; m < 4; m++) d[m][v] = d[m][v] + __fmul_rn(p0, gm[m - 1][v]);
+          d[4][v] = d[4][v] + __fmul_rn(e0, ug);
         }
       }
       if (sponge) {
