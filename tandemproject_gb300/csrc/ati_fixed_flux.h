@@ -1,81 +1,21 @@
 // ati_fixed_flux.h — the FP64 fast path's fluxes at one point in 64-bit fixed point (see ati_fixed.h for why).
 //
-// A group of inputs that enter sums together (the nine metrics, the velocity derivatives, the temperature derivatives,
-// the velocities, ...) shares one exponent, its largest; an input becomes a signed integer below 2^60 in that unit.
-// Sums of products run in integers (three 32 x 32 + 64 bit multiply-adds a product, the lowest partial product left
-// out); sums over groups align to the larger unit first.  A flux component's error before its one rounding is some
-// 2^-56 of the largest term that enters it, where FP64 rounds each of some ten operations at 2^-53: against extended
-// precision, 0.4 to 0.8 of the FP64 arithmetic's error on flows at rest, slow and fast, equal where a component is a
-// single product.
+// Every operand is an integer just below 2^60 times its own power of two, whatever the others' sizes: along a stretched
+// grid the metrics of two directions differ by a thousand, and a small velocity component has its own accuracy.  Sums of
+// products run in integers (three 32 x 32 + 64 bit multiply-adds a product, the lowest partial product left out), each
+// product aligned to the sum's largest.  A sum's error is some 2^-57 of its largest term, where FP64 rounds each operation
+// at 2^-53.  Measured against extended precision in units of the terms that make a component up, over metric ratios of 1
+// to 10^6, velocity components 1 to 10^-30 of the largest, derivatives of all sizes: 0.49 to 0.80 of the FP64 arithmetic's
+// error, inviscid momentum 0.84 to 1.001 (correctly rounded there but for 2^-57).
 //
-// The fluxes are formed as tensors in space and then contracted with the metrics (src/Main3D.f90:631-766):
-//   rho V,  (rho u_m) V_k + p delta - tau,  (rhoE + p) V - p u_inf - r2 grad T - u . tau,   V = u + u_inf
+// As the FP64 kernels do (src/Main3D.f90:631-766): contravariant velocities S_n = M_n . (u + u_inf), then along n
+//   rho S,  (rho u_m) S + M . (p delta - tau)_m,  (rhoE + p) S + M . w,   w = u . (-tau) - r2 grad T - p u_inf
 #pragma once
-#include <cstdint>
-#include <cstring>
+#include "ati_fixed_num.h"
 
 namespace ati {
 
-#ifdef __CUDACC__
-#define ATI_HD __host__ __device__ __forceinline__
-#else
-#define ATI_HD inline
-#endif
-
 namespace fxf {
-
-using i64 = long long;
-using u64 = unsigned long long;
-
-ATI_HD i64 mad_wide(int a, int b, i64 c) {
-#ifdef __CUDA_ARCH__
-  i64 r;
-  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-  return r;
-#else
-  return (i64)((u64)((i64)a * b) + (u64)c);
-#endif
-}
-ATI_HD int hi_word(double f) {
-#ifdef __CUDA_ARCH__
-  return __double2hiint(f);
-#else
-  u64 b;
-  std::memcpy(&b, &f, 8);
-  return (int)(b >> 32);
-#endif
-}
-ATI_HD unsigned lo_word(double f) {
-#ifdef __CUDA_ARCH__
-  return (unsigned)__double2loint(f);
-#else
-  u64 b;
-  std::memcpy(&b, &f, 8);
-  return (unsigned)b;
-#endif
-}
-ATI_HD double from_words(int hi, unsigned lo) {
-#ifdef __CUDA_ARCH__
-  return __hiloint2double(hi, (int)lo);
-#else
-  const u64 b = (u64)(unsigned)hi << 32 | lo;
-  double f;
-  std::memcpy(&f, &b, 8);
-  return f;
-#endif
-}
-ATI_HD int imax(int a, int b) { return a > b ? a : b; }
-ATI_HD int imin(int a, int b) { return a < b ? a : b; }
-ATI_HD unsigned umax(unsigned a, unsigned b) { return a > b ? a : b; }
-
-// a 64-bit value as hi 2^32 + lo, both signed
-struct Split {
-  int hi, lo;
-};
-ATI_HD Split split(i64 x) {
-  const int lo = (int)(unsigned)x;
-  return {(int)(x >> 32) + (int)((unsigned)lo >> 31), lo};
-}
 
 // a sum of products of fixed-point values, in units of 2^64 of the product's; value(K): in units of 2^(64-K)
 struct Dot {
@@ -89,191 +29,142 @@ struct Dot {
   ATI_HD i64 value(int K = 0) const { return (i64)((u64)hi << K) + (mid >> (32 - K)); }
 };
 
-// exponents: a group's exponent e (biased, of its largest value) is kept in [E_MIN, E_MAX]; smaller groups lose what
-// lies 60 bits below 2^-200, and a point with a larger or non-finite value is left to the FP64 arithmetic
-constexpr int E_MIN = 1023 - 200, E_MAX = 1023 + 200;
-constexpr int BITS = 60;
-// |x| < 2^60, x 2^(unit) the value
-ATI_HD int unit(int e) { return e - 1023 - (BITS - 1); }
-ATI_HD unsigned mag(double f) { return (unsigned)hi_word(f) & 0x7fffffffu; }
-ATI_HD i64 conv(double f, int e) {
-  const int h = hi_word(f), r = imin(e - ((h >> 20) & 0x7ff), 63);
-  const u64 m = (((u64)((unsigned)h & 0xfffffu) | 0x100000u) << 32 | lo_word(f)) << (BITS - 53);
+// an operand: x 2^e
+struct Num {
+  i64 x;
+  int e;
+};
+
+// Inputs with an exponent above E_MAX (infinities and NaNs among them) leave the point to the FP64 arithmetic: products of
+// five inputs stay in FP64's range.  Results below FP64's normal range are zero.
+constexpr int E_MAX = 1023 + 200;
+// a double as it is: 2^59 <= |x| < 2^60, but for subnormals and zero (x = 0)
+ATI_HD Num num(double f) {
+  const int h = hi_word(f), g = (h >> 20) & 0x7ff;
+  const u64 m = ((u64)(((unsigned)h & 0xfffffu) | (g ? 0x100000u : 0u)) << 32 | lo_word(f)) << 7;
   const i64 s = (i64)(h >> 31);
-  return ((i64)(m >> r) ^ s) - s;
+  return {((i64)m ^ s) - s, imax(g, 1) - 1023 - 59};
 }
-// x 2^u as a double (x = 0: zero)
-ATI_HD double to_double(i64 x, int u) {
-  const double d = (double)x;
-  const int h = hi_word(d);
-  return from_words(h == 0 ? 0 : h + u * (1 << 20), lo_word(d));
+ATI_HD double to_double(Num a) {
+  const double d = (double)a.x;
+  const int h = hi_word(d), m = (h & 0x7fffffff) + imax(a.e, -2000) * (1 << 20);
+  return m < (1 << 20) || a.x == 0 ? 0.0 : from_words(m | (h & (int)0x80000000), lo_word(d));
 }
-ATI_HD i64 shr(i64 x, int s) { return x >> imin(s, 63); }
+// |x| < 2^60 moved up to 2^59 and above (a value below 2^32 by 28 bits)
+ATI_HD Num norm(Num a) {
+  const int h = (int)(a.x >> 32), s = imax(clz((unsigned)(h ^ (h >> 31))) - 4, 0);
+  return {(i64)((u64)a.x << s), a.e - s};
+}
+// a sum of N <= 5 products of operands below 2^60, each aligned to the largest: below 2^60
+template <int N>
+ATI_HD Num dot(const Num (&a)[N], const Num (&b)[N]) {
+  constexpr int K = N == 1 ? 4 : (N == 2 ? 3 : (N <= 4 ? 2 : 1));
+  int E = a[0].e + b[0].e;
+#pragma unroll
+  for (int k = 1; k < N; k++) E = imax(E, a[k].e + b[k].e);
+  Dot d;
+  d.mid = (i64)1 << (31 - K);  // (to the nearest)
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const Split u = split(N == 1 ? a[k].x : shr(a[k].x, E - a[k].e - b[k].e)), v = split(b[k].x);
+    d.add(u, v);
+    if (N == 2) d.mid += mad_wide(u.lo, v.lo, (i64)1 << 31) >> 32;
+  }
+  return {d.value(K), E + 64 - K};
+}
+ATI_HD Num mul(Num a, Num b) { return dot<1>({a}, {b}); }
 
 }  // namespace fxf
 
 // one point's inputs: metrics m[direction][component], derivatives dv[field u v w T][direction], velocity, pressure,
 // state, r1 = mu J (the viscosity times the Jacobian), r2 = r1 / ((gamma - 1) Pr), frame velocity
-struct FluxIn {
+struct FixFluxIn {
   double m[3][3], dv[4][3], vel[3], p, q[5], r1, r2, umf[3];
 };
 
 // F[c * 3 + n]: component c of the flux along direction n; false (F not set) for a point left to the FP64 arithmetic
 template <bool VISC>
-ATI_HD bool flux_point_fixed(const FluxIn &I, double *F) {
+ATI_HD bool flux_point_fixed(const FixFluxIn &I, double *F) {
   using namespace fxf;
-  unsigned gm = 0, gv = 0, gq = 0, gd = 0, gt = 0;
+  unsigned all = umax(mag(I.p), umax(mag(I.q[0]), mag(I.q[4])));
 #pragma unroll
-  for (int n = 0; n < 3; n++)
+  for (int n = 0; n < 3; n++) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) gm = umax(gm, mag(I.m[n][k]));
+    for (int k = 0; k < 3; k++) all = umax(all, mag(I.m[n][k]));
+    all = umax(all, umax(mag(I.q[1 + n]), umax(mag(I.vel[n]), mag(I.umf[n]))));
+    if (VISC)
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    gv = umax(gv, umax(mag(I.vel[k]), mag(I.umf[k])));
-    gq = umax(gq, mag(I.q[1 + k]));
+      for (int f = 0; f < 4; f++) all = umax(all, mag(I.dv[f][n]));
   }
-  const unsigned gr = mag(I.q[0]), gp = umax(mag(I.p), mag(I.q[4]));
-  unsigned all = umax(umax(gm, gv), umax(umax(gq, gr), gp));
-  if (VISC) {
-#pragma unroll
-    for (int n = 0; n < 3; n++) {
-      gd = umax(umax(gd, mag(I.dv[0][n])), umax(mag(I.dv[1][n]), mag(I.dv[2][n])));
-      gt = umax(gt, mag(I.dv[3][n]));
-    }
-    all = umax(all, umax(umax(gd, gt), umax(mag(I.r1), mag(I.r2))));
-  }
+  if (VISC) all = umax(all, umax(mag(I.r1), mag(I.r2)));
   if ((int)(all >> 20) > E_MAX) return false;
-  auto expo = [](unsigned g) { return imax((int)(g >> 20), E_MIN); };
-  const int em = expo(gm), ev = expo(gv), eq = expo(gq), er = expo(gr), ep = expo(gp);
-  const int um = unit(em), uv = unit(ev);
-  Split M[3][3];
+  Num M[3][3];
 #pragma unroll
   for (int n = 0; n < 3; n++)
 #pragma unroll
-    for (int k = 0; k < 3; k++) M[n][k] = split(conv(I.m[n][k], em));
-  // velocities in the moving frame
-  Split vel[3], umf[3], V[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const i64 a = conv(I.vel[k], ev), b = conv(I.umf[k], ev);
-    vel[k] = split(a);
-    umf[k] = split(-b);
-    V[k] = split(a + b);
-  }
-  auto contract = [&](const Split *G, int ug, double *f) {
-#pragma unroll
-    for (int n = 0; n < 3; n++) {
-      Dot d;
-#pragma unroll
-      for (int k = 0; k < 3; k++) d.add(M[n][k], G[k]);
-      f[n] = to_double(d.value(3), um + ug + 61);
-    }
-  };
-  Split G[3];
-  {  // mass
-    const Split r = split(conv(I.q[0], er));
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      Dot d;
-      d.add(r, V[k]);
-      G[k] = split(d.value(3));
-    }
-    contract(G, unit(er) + uv + 61, F);
-  }
-  const i64 p = conv(I.p, ep);
-  // viscous stresses t: xx yy zz xy yz zx in units of 2^ut; heat flux r2 grad T
-  i64 t[6] = {0, 0, 0, 0, 0, 0}, hq[3] = {0, 0, 0};
-  int ut = 0, uh = 0;
+    for (int k = 0; k < 3; k++) M[n][k] = num(I.m[n][k]);
+  // minus the stresses, t: xx yy zz xy yz zx, and w = u . t - r2 grad T - p u_inf
+  Num t[6], w[3];
+  const Num p = num(I.p);
   if (VISC) {
-    const int ed = expo(gd), et = expo(gt), e1 = expo(mag(I.r1)), e2 = expo(mag(I.r2));
-    auto grad = [&](int f, int e, int up, i64 *c) {
-      Split d[3];
-#pragma unroll
-      for (int n = 0; n < 3; n++) d[n] = split(conv(I.dv[f][n], e));
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        Dot s;
-#pragma unroll
-        for (int n = 0; n < 3; n++) s.add(M[n][k], d[n]);
-        c[k] = s.value(up);
-      }
+    auto grad = [&](int f, int k) {
+      return dot<3>({M[0][k], M[1][k], M[2][k]}, {num(I.dv[f][0]), num(I.dv[f][1]), num(I.dv[f][2])});
     };
-    i64 u[3], v[3], w[3], T[3];
-    grad(0, ed, 2, u);
-    grad(1, ed, 2, v);
-    grad(2, ed, 2, w);
-    grad(3, et, 4, T);
-    // two thirds of the divergence: 2/3 = 0x2AAAAAAA.AAAAAAAA 2^-30
-    const Split dv = split(u[0] + v[1] + w[2]);
-    i64 mid = mad_wide(0x2aaaaaab, dv.lo, (i64)1 << 29);
-    mid = mad_wide(-0x55555555, dv.hi, mid);
-    const i64 d5 = (mad_wide(0x2aaaaaab, dv.hi, 0) << 2) + (mid >> 30);
-    const Split r1 = split(conv(I.r1, e1)), r2 = split(conv(I.r2, e2));
-    auto scaled = [&](Split r, i64 x) {
-      Dot s;
-      s.add(r, split(x));
-      return s.value(2);
+    const Num r1 = num(-I.r1), r1t = num(-I.r1 * (2.0 / 3.0)), r2 = num(-I.r2);
+    const Num ux = grad(0, 0), vy = grad(1, 1), wz = grad(2, 2);
+    {  // 2 u_x - 2/3 div u = 2/3 (2 u_x - v_y - w_z)
+      const int E = imax(ux.e, imax(vy.e, wz.e)) + 2;
+      const i64 a = shr(ux.x, E - ux.e), b = shr(vy.x, E - vy.e), c = shr(wz.x, E - wz.e);
+      t[0] = mul(r1t, norm({2 * a - b - c, E}));
+      t[1] = mul(r1t, norm({2 * b - a - c, E}));
+      t[2] = mul(r1t, norm({2 * c - a - b, E}));
+    }
+    auto shear = [&](Num a, Num b) {
+      const int E = imax(a.e, b.e) + 1;
+      return mul(r1, norm({shr(a.x, E - a.e) + shr(b.x, E - b.e), E}));
     };
-    t[0] = scaled(r1, 2 * u[0] - d5);
-    t[1] = scaled(r1, 2 * v[1] - d5);
-    t[2] = scaled(r1, 2 * w[2] - d5);
-    t[3] = scaled(r1, v[0] + u[1]);
-    t[4] = scaled(r1, w[1] + v[2]);
-    t[5] = scaled(r1, u[2] + w[0]);
-    ut = unit(e1) + um + unit(ed) + 62 + 62;
+    t[3] = shear(grad(1, 0), grad(0, 1));
+    t[4] = shear(grad(2, 1), grad(1, 2));
+    t[5] = shear(grad(0, 2), grad(2, 0));
+    const Num u[3] = {num(I.vel[0]), num(I.vel[1]), num(I.vel[2])};
+    const int at[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
 #pragma unroll
-    for (int k = 0; k < 3; k++) hq[k] = scaled(r2, T[k]);
-    uh = unit(e2) + um + unit(et) + 60 + 62;
+    for (int k = 0; k < 3; k++)
+      w[k] = norm(dot<5>({t[at[k][0]], t[at[k][1]], t[at[k][2]], norm(grad(3, k)), num(-I.umf[k])}, {u[0], u[1], u[2], r2, p}));
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; k++) w[k] = mul(p, num(-I.umf[k]));
   }
-  {  // momentum: q_m V_k + p delta - tau
-    const int us = VISC ? imax(unit(ep), ut) : unit(ep), uq = unit(eq) + uv + 61, uP = imax(us, uq);
-    const int sp = uP - unit(ep), st = uP - ut, sq = uP - uq;
-    const i64 pp = shr(p, sp);
-    i64 ts[6];
+  // contravariant velocities in the moving frame
+  Num S[3];
+  {
+    const Num V[3] = {num(I.vel[0] + I.umf[0]), num(I.vel[1] + I.umf[1]), num(I.vel[2] + I.umf[2])};
+#pragma unroll
+    for (int n = 0; n < 3; n++) S[n] = norm(dot<3>({M[n][0], M[n][1], M[n][2]}, {V[0], V[1], V[2]}));
+  }
+  const Num r = num(I.q[0]);
+#pragma unroll
+  for (int n = 0; n < 3; n++) F[n] = to_double(mul(r, S[n]));
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    const Num q = num(I.q[1 + m]);
     if (VISC) {
+      const int E = imax(p.e, t[m].e) + 1;
+      const Num s = {shr(p.x, E - p.e) + shr(t[m].x, E - t[m].e), E};
+      const Num row[3] = {m == 0 ? s : (m == 1 ? t[3] : t[5]), m == 0 ? t[3] : (m == 1 ? s : t[4]),
+                          m == 0 ? t[5] : (m == 1 ? t[4] : s)};
 #pragma unroll
-      for (int k = 0; k < 6; k++) ts[k] = shr(t[k], st);
-    }
+      for (int n = 0; n < 3; n++)
+        F[3 * (m + 1) + n] = to_double(dot<4>({S[n], M[n][0], M[n][1], M[n][2]}, {q, row[0], row[1], row[2]}));
+    } else {
 #pragma unroll
-    for (int m = 0; m < 3; m++) {
-      const Split q = split(conv(I.q[1 + m], eq));
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        Dot d;
-        d.add(q, V[k]);
-        i64 x = shr(d.value(3), sq);
-        if (m == k) x += pp;
-        if (VISC) x -= ts[m == k ? m : (m + k == 1 ? 3 : (m + k == 3 ? 4 : 5))];
-        G[k] = split(x);
-      }
-      contract(G, uP, F + 3 * (m + 1));
+      for (int n = 0; n < 3; n++) F[3 * (m + 1) + n] = to_double(dot<2>({S[n], M[n][m]}, {q, p}));
     }
   }
-  {  // energy: (rhoE + p) V - p u_inf - r2 grad T - u . tau
-    const Split h = split(conv(I.q[4], ep) + p), ps = split(p);
-    const int ua = unit(ep) + uv + 62, uc = VISC ? uv + ut + 62 : 0;
-    const int uE = VISC ? imax(ua, imax(uh, uc)) : ua;
-    Split ts[6];
-    if (VISC) {
+  const Num h = num(I.q[4] + I.p);
 #pragma unroll
-      for (int k = 0; k < 6; k++) ts[k] = split(t[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      Dot d;
-      d.add(h, V[k]);
-      d.add(ps, umf[k]);
-      i64 x = shr(d.value(2), uE - ua);
-      if (VISC) {
-        Dot c;
-#pragma unroll
-        for (int j = 0; j < 3; j++) c.add(vel[j], ts[j == k ? j : (j + k == 1 ? 3 : (j + k == 3 ? 4 : 5))]);
-        x -= shr(hq[k], uE - uh) + shr(c.value(2), uE - uc);
-      }
-      G[k] = split(x);
-    }
-    contract(G, uE, F + 12);
-  }
+  for (int n = 0; n < 3; n++)
+    F[12 + n] = to_double(dot<4>({S[n], M[n][0], M[n][1], M[n][2]}, {h, w[0], w[1], w[2]}));
   return true;
 }
 

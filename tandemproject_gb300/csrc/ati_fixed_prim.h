@@ -14,16 +14,6 @@ namespace fxf {
 // density and energy from 2^-100 up (below, a state is not a flow's: FP64 operations)
 constexpr int E_STATE_MIN = 1023 - 100;
 
-// a constant as a normalised significand (2^59 <= |x| < 2^60) and its unit
-struct Num {
-  Split x;
-  int u;
-};
-ATI_HD Num num(double f) {
-  const int e = (int)(mag(f) >> 20);
-  return {split(conv(f, e)), unit(e)};
-}
-
 ATI_HD float approx_rcp(float x) {
 #ifdef __CUDA_ARCH__
   float y;
@@ -67,23 +57,24 @@ ATI_HD i64 seed60(float f) {
 }
 
 // a product in units of 2^(64-K) of the product's
-ATI_HD i64 mul(Split a, Split b, int K) {
+ATI_HD i64 prod(Split a, Split b, int K) {
   Dot d;
   d.add(a, b);
   return d.value(K);
 }
 
-// 1/f for a positive normal f: x in (2^59, 2^60], 1/f = x 2^(-60 - (e - 1023)) with e the biased exponent of f
-ATI_HD Split recip(double f) {
+// 1/f for a positive normal f, its x in (2^59, 2^60]
+ATI_HD Num recip(double f) {
   const int h = hi_word(f);
-  const Split a = split(conv(f, (h >> 20) & 0x7ff));  // 2^59 times the significand
+  const Num n = num(f);
+  const Split a = split(n.x);  // 2^59 times the significand
   i64 x = seed60(approx_rcp(float_of(0x3f800000u | (((unsigned)h & 0xfffffu) << 3) | (lo_word(f) >> 29))));
 #pragma unroll
   for (int it = 0; it < 2; it++) {
     const Split s = split(x);
-    x += mul(s, split(((i64)1 << 62) - mul(a, s, 7)), 2);
+    x += prod(s, split(((i64)1 << 62) - prod(a, s, 7)), 2);
   }
-  return split(x);
+  return {x, -119 - n.e};  // (2^59 2^60 over the significand's integer)
 }
 
 }  // namespace fxf
@@ -102,52 +93,39 @@ ATI_HD bool prim_point_fixed(const PrimFx &C, const double q[5], double out[6]) 
   using namespace fxf;
   const unsigned gr = (unsigned)hi_word(q[0]), ge = (unsigned)hi_word(q[4]);  // (a negative value: beyond E_MAX)
   const unsigned gq = umax(mag(q[1]), umax(mag(q[2]), mag(q[3])));
-  const int er = (int)(gr >> 20), ee = (int)(ge >> 20), eq = imax((int)(gq >> 20), E_MIN);
-  if ((int)(umax(gr, umax(ge, gq)) >> 20) > E_MAX || imin(er, ee) < E_STATE_MIN) return false;
-  const Split r = recip(q[0]);
-  const int ur = -60 - (er - 1023), uq = unit(eq);
-  const int uv = uq + ur + 60;
-  Dot kin;
+  if ((int)(umax(gr, umax(ge, gq)) >> 20) > E_MAX || (int)(umin(gr, ge) >> 20) < E_STATE_MIN) return false;
+  const Num r = recip(q[0]);
+  const Num m[3] = {num(q[1]), num(q[2]), num(q[3])};
+  const Num v[3] = {mul(m[0], r), mul(m[1], r), mul(m[2], r)};
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const int e = imax((int)(mag(q[1 + k]) >> 20), E_MIN), s = eq - e;  // each velocity in its own unit
-    const i64 m = conv(q[1 + k], e), v = mul(split(m), r, 4);
-    out[k] = to_double(v, uv - s);
-    kin.add(split(shr(m, s)), split(shr(v, s)));
-  }
+  for (int k = 0; k < 3; k++) out[k] = to_double(v[k]);
   // rhoE - rho u . u / 2 in the larger unit
-  const int ue = unit(ee), uk = uq + uv + 61, up = imax(ue, uk);
-  const i64 d = shr(conv(q[4], ee), up - ue) - shr(kin.value(2), up - uk);
+  const Num E = num(q[4]), kin = dot<3>({m[0], m[1], m[2]}, {v[0], v[1], v[2]});
+  const int up = imax(E.e, kin.e - 1);
+  const i64 d = shr(E.x, up - E.e) - shr(kin.x, up - (kin.e - 1));
   if (d <= 0) return false;
-  // (a constant's significand at 2^59.. of 2^60: the product keeps the unit's bits)
-  const i64 p = mul(split(d), C.gamm1.x, 4);
-  const int u1 = up + C.gamm1.u + 60;
-  out[4] = to_double(p, u1);
-  const i64 gp = mul(split(p), C.gam.x, 4);
-  const i64 t = mul(split(gp), r, 4);
-  const double T = to_double(t, u1 + C.gam.u + 60 + ur + 60);
+  const Num p = mul(Num{d, up}, C.gamm1);
+  out[4] = to_double(p);
+  const Num t = mul(mul(p, C.gam), r);
+  const double T = to_double(t);
   out[3] = T;
   const int et = (int)(mag(T) >> 20);
-  if (t <= 0) return false;
+  if (t.x <= 0) return false;
   // sqrt(T) = a y, a = T 2^-2j in [1, 4): y = 1/sqrt(a)
   const int odd = (et - 1023) & 1;
-  const i64 a58 = conv(T, et) >> (1 - odd);  // 2^58 a
+  const Num tn = num(T);
+  const i64 a58 = tn.x >> (1 - odd);  // 2^58 a
   const Split a = split(a58);
   const unsigned fb = (((unsigned)hi_word(T) & 0xfffffu) << 3) | (lo_word(T) >> 29);
   i64 y = seed60(approx_rsqrt(float_of((0x3f800000u + ((unsigned)odd << 23)) | fb)));
 #pragma unroll
   for (int it = 0; it < 2; it++) {
     const Split s = split(y);
-    const Split y2 = split(mul(s, s, 4));
-    y += mul(s, split(((i64)1 << 62) - mul(a, y2, 8)), 1);
+    const Split y2 = split(prod(s, s, 4));
+    y += prod(s, split(((i64)1 << 62) - prod(a, y2, 8)), 1);
   }
-  const i64 root = mul(a, split(y), 4);  // 2^58 sqrt(a), below 2^59
-  const double ts = T + C.s;
-  const Split rs = recip(ts);
-  const int es = (int)(mag(ts) >> 20);
-  const i64 tt = mul(split(conv(T, et)), split(root), 4);                 // T sqrt(a)
-  const i64 x = mul(split(mul(split(tt), rs, 4)), C.c.x, 4);
-  out[5] = to_double(x, unit(et) + (-58 + ((et - 1023 - odd) >> 1)) + 60 + (-60 - (es - 1023)) + 60 + C.c.u + 60);
+  const Num root = {prod(a, split(y), 4), -58 + ((et - 1023 - odd) >> 1)};  // sqrt(T), its x below 2^59
+  out[5] = to_double(mul(mul(mul(tn, root), recip(T + C.s)), C.c));
   return true;
 }
 

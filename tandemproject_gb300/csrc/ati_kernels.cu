@@ -1918,8 +1918,8 @@ __device__ __forceinline__ bool prim_point(const Eng<R> &e, const PrimConst<R> &
 }
 
 // the FP64 fast path's primitives in fixed point (prim_point_fixed); states that leave its range, or are not physical,
-// take the FP64 operations.  On 8.85 M points 569 -> 235 us a launch (88 B a point, 3.3 TB/s) against the FP64 kernel,
-// which the FP64 pipe bound at some 37 operations a point; two to four CTAs an SM measure the same.
+// take the FP64 operations.  On 8.85 M points 569 -> 257 us a launch (88 B a point, 3.0 TB/s) against the FP64 kernel,
+// which the FP64 pipe bound at some 37 operations a point; integer issue bounds this one.
 __device__ __noinline__ bool prim_point_fp64(const Eng<double> &e, const PrimConst<double> &C, int64_t g,
                                              const double q[5]) {
   return prim_point<double>(e, C, e.N, g, q);
@@ -2328,20 +2328,23 @@ __global__ void __launch_bounds__(256, Freestream<R>::on ? 5 : 1) k_flux(Eng<R> 
 
 // the FP64 fast path's fluxes in fixed point (flux_point_fixed), the viscous ones with the stresses at the point (no
 // stress plane is written or read); points whose values leave its range take the FP64 operations.  On 8.85 M points
-// 2131 -> 830 us a launch against the FP64 kernel, whose 138 operations a point kept the FP64 pipe 91 % busy; 376 B a
-// point, 4.0 TB/s.  Two CTAs of 256 threads an SM, 128 registers: one CTA (255 registers) 959 us, three (85) 1060 us.
+// 2131 -> 1122 us a launch against the FP64 kernel, whose 138 operations a point kept the FP64 pipe 91 % busy; 376 B a
+// point, 3.0 TB/s: integer issue bounds it, some 115 products a point, each aligned to its sum's largest.  (With one
+// exponent for all operands of a kind instead of each its own it took 830 us, but held the smaller ones in fewer bits
+// than FP64.)  Three CTAs of 128 threads an SM, 168 registers: two of 256 (128) 1143 us, one (255) 1270, four of 128 1232.
 template <bool VISC>
 __device__ __noinline__ void flux_point_fp64(const Eng<double> &e, int64_t g, double u1, double u2, double u3,
                                              const ViscConst<double> &V) {
   flux_fast_point<VISC, VISC>(e, e.N, g, u1, u2, u3, &V);
 }
+constexpr int FLUX_FIXED_THREADS = 128;
 template <bool VISC>
-__global__ void __launch_bounds__(256, 2) k_flux_fixed(const __grid_constant__ Eng<double> e) {
+__global__ void __launch_bounds__(FLUX_FIXED_THREADS, 3) k_flux_fixed(const __grid_constant__ Eng<double> e) {
   const int64_t N = e.N;
   TILE_LOOP(e, T) {
     const Scheme &S = e.sc[T.cs];
     const Scalars &SC = e.scal[T.cs];
-    FluxIn I;
+    FixFluxIn I;
     I.umf[0] = SC.umf[1];
     I.umf[1] = SC.umf[2];
     I.umf[2] = SC.umf[3];
@@ -3396,8 +3399,8 @@ static void pointwise_t(const Eng<R> &eng, cudaStream_t st, int which) {
     case PW_FLUX:
     case PW_FLUX_STRESS:
       if constexpr (kFast && !Freestream<R>::on) {  // (the stresses at the point, whether or not k_visc wrote its planes)
-        if (e.fx_flux == 1) k_flux_fixed<true><<<g, t, 0, st>>>(e);
-        else if (e.fx_flux == 2) k_flux_fixed<false><<<g, t, 0, st>>>(e);
+        if (e.fx_flux == 1) k_flux_fixed<true><<<g, FLUX_FIXED_THREADS, 0, st>>>(e);
+        else if (e.fx_flux == 2) k_flux_fixed<false><<<g, FLUX_FIXED_THREADS, 0, st>>>(e);
         if (e.fx_flux) break;
       }
       if (which == PW_FLUX) {
