@@ -25,6 +25,7 @@ SOURCES = [
     ("ati_kernels.cu", "ati_kernels_fast.o", ["-DATI_KNS=fast", "-DATI_KFAST=1", "-fmad=true"]),
     ("ati_kernels.cu", "ati_kernels_strict.o", ["-DATI_KNS=strict", "-DATI_KFAST=0", "-fmad=false"]),
     ("ati_fixed.cu", "ati_fixed.o", []),
+    ("ati_fixed_tab.cpp", "ati_fixed_tab.o", []),
     ("ati_api.cu", "ati_api.o", ["-fmad=false"]),
     ("ati_scheme.cpp", "ati_scheme.o", []),
     ("ati_probe.cu", "ati_probe.o", []),

@@ -76,6 +76,12 @@ struct ati_handle {
   }
   std::vector<PTile> hpt;
   std::vector<LTile> hlt[4];
+  // fixed-point line sweeps of an FP64 handle, [derivative, filter] (ati_fixed.h): scales, tables (on the host until the
+  // handle is made), and per direction the blocks whose lines they take
+  FixOp fix_op[2];
+  std::vector<int> fix_rows[2];
+  std::vector<int64_t> fix_ends[2];
+  std::vector<char> fix_blk[4];
   std::vector<LTile> hlts[4];  // tiles of the segmented sweeps (mixed path), by class (segc)
   SegClass segc[4][SEG_NCLASS] = {};
   int nsegc[4] = {0, 0, 0, 0};
@@ -486,11 +492,11 @@ static void make_tiles(ati_handle *h, int sg2, int sg3, int pt) {
   for (int nn = 1; nn <= 3; nn++) {
     h->hlt[nn].clear();
     const int step = nn == 1 ? XC_NL : (nn == 2 ? sg2 : sg3);
-    // (blocks whose lines the fixed-point sweeps can take come first: those sweeps leave the tiles from nlt_fx on)
+    // (blocks whose lines the fixed-point sweeps take come first: those sweeps leave the tiles from nlt_fx on)
     for (int other = 0; other <= 1; other++) {
       for (int gb = 0; gb < h->nb; gb++) {
         const BlockDev &B = h->blk[gb];
-        if (fx_line((nn == 1 ? B.lxi : (nn == 2 ? B.let : B.lze)) + 1) != (other == 0)) continue;
+        if (h->fix_blk[nn][gb] != (other == 0)) continue;
         for (int t0 = 0; t0 < B.nbsize[nn]; t0 += step) h->hlt[nn].push_back(LTile{gb, t0});
       }
       if (!other) h->ed.nlt_fx[nn] = (int)h->hlt[nn].size();
@@ -588,6 +594,8 @@ static int encode_tmaps(ati_handle *h, std::vector<TmaMap> &out) {
     }
   return ATI_OK;
 }
+
+static void fix_tables(ati_handle *h, const std::vector<double> &facd, const std::vector<double> &facf);
 
 static int build_tables(ati_handle *h, std::vector<double> &facd, std::vector<double> &facf, std::vector<double> &spg) {
   int64_t off = 0, face = 0, fac = 0;
@@ -717,6 +725,7 @@ static int build_tables(ati_handle *h, std::vector<double> &facd, std::vector<do
     r.n++;
     r.maxline = std::max(r.maxline, T[h->tl_force.off + q].nline);
   }
+  fix_tables(h, facd, facf);
   // work queues, at their finest tiles (the device arrays are sized for these)
   make_tiles(h, SG_MIN, SG_MIN, PT_MIN);
   h->max_pt = h->hpt.size();
@@ -732,7 +741,7 @@ static int build_tables(ati_handle *h, std::vector<double> &facd, std::vector<do
     auto len = [&](const BlockDev &B) { return nn == 1 ? B.lxi + 1 : (nn == 2 ? B.let + 1 : B.lze + 1); };
     std::vector<int> counts;
     // (an FP64 handle's classes are the fixed-point sweeps': without the lines they do not take)
-    auto in = [&](int gb) { return h->mixed || fx_line(len(h->blk[gb])); };
+    auto in = [&](int gb) { return h->mixed || h->fix_blk[nn][gb]; };
     for (int gb = 0; gb < h->nb; gb++)
       if (in(gb)) counts.push_back(seg_count(len(h->blk[gb])));
     std::sort(counts.begin(), counts.end());
@@ -920,281 +929,35 @@ static void fu_tables(const ati_handle *h, const std::vector<double> &fac, doubl
   }
 }
 
-// Tables of the fixed-point line sweeps (ati_fixed.h) of one operator (filt: the filter, else the derivative).
-// The rows as linear forms in the line's values are built once per kind of line (one-sided ends, or periodic onto
-// its own block) on a line of 56 points, two segments; their amplification of the line's largest neighbour
-// difference (the sum of the magnitudes of a row's suffix sums; a periodic line also by the difference across its
-// ends) bounds every value a solve holds, whatever the line's length: away from the ends the rows repeat.  From it
-// and the coefficients come the operator's extra scale 2^k and the bits gbits a scaled difference may take.
-struct FixTables {
-  bool ok[4] = {false, false, false, false};
-  int gbits = 0, k = 0;
-  std::vector<int> rows;
-  std::vector<int64_t> ends;
-};
-
-namespace {
-// right-hand-side rows 0-2 of a line end as weights on its first seven points (one-sided ends)
-void end_weights(const Scheme &S, bool filt, double E[3][7]) {
-  std::memset(E, 0, sizeof(double) * 21);
-  if (!filt) {
-    for (int r = 0; r < 3; r++)
-      for (int q = 0, n = 0; q < 7; q++) {
-        if (q == r) continue;
-        E[r][q] += S.abc[r][n];
-        E[r][r] -= S.abc[r][n];
-        n++;
-      }
-    return;
+// The fixed-point line sweeps (ati_fixed.h) of an FP64 handle: their tables, and the blocks whose lines they take in each
+// direction.
+static void fix_tables(ati_handle *h, const std::vector<double> &facd, const std::vector<double> &facf) {
+  for (int nn = 1; nn <= 3; nn++) h->fix_blk[nn].assign(h->nb, 0);
+  if (h->cfg.precision != ATI_FP64) return;
+  for (int q = 0; q < 2; q++) {
+    h->fix_op[q] = fix_operator(h->sh, q == 1);
+    h->fix_rows[q].assign((size_t)(h->nfac + 2 * FX_PAD) * FX_RT, 0);
+    h->fix_ends[q].assign((size_t)h->nb * 3 * FX_ET, 0);
   }
-  // the extrapolated points rv(n) = w0 - ffx(n) sum_q fex(q) (w(q) - w0) of src/Subroutines3D.f90:160-170
-  double rv[4][7];
-  std::memset(rv, 0, sizeof(rv));
-  for (int n = 1; n <= 3; n++) {
-    rv[n][0] = 1.0;
-    for (int q = 1; q <= 3; q++) {
-      rv[n][q] -= S.ffx[n] * S.fex[q];
-      rv[n][0] += S.ffx[n] * S.fex[q];
-    }
-  }
-  auto pt = [&](int r, double c, int at) {  // c times point at of the line (negative: extrapolated)
-    if (at >= 0) E[r][at] += c;
-    else
-      for (int q = 0; q < 7; q++) E[r][q] += c * rv[-at][q];
-  };
-  for (int r = 0; r < 3; r++) {
-    const double c[3] = {S.fam[r], S.fbm[r], S.fcm[r]};
-    for (int d = 1; d <= 3; d++) {
-      pt(r, c[d - 1], r - d);
-      pt(r, c[d - 1], r + d);
-      pt(r, -2.0 * c[d - 1], r);
-    }
-  }
-}
-
-// the largest sum of magnitudes of the row's weights on neighbour differences
-double amplitude(const std::vector<double> &c, bool per) {
-  const int L = (int)c.size();
-  double best = 0, s = 0;
-  for (int j = L - 1; j >= 1; j--) best += std::fabs(s += c[j]);
-  if (!per) return best;
-  for (int m = L / 8; m < L - 1; m += L / 8) {  // points up to m reached from point 0, the others from the far end
-    double t = 0, v = 0;
-    for (int j = m; j >= 1; j--) t += std::fabs(v += c[j]);
-    v = 0;
-    for (int j = m + 1; j < L - 1; j++) t += std::fabs(v += c[j]);
-    best = std::min(best, t + std::fabs(v + c[L - 1]));
-  }
-  return best;
-}
-}  // namespace
-
-static void fix_tables(const ati_handle *h, bool filt, const std::vector<double> &fac, FixTables &T) {
-  const Scheme &S = h->sh.s;
-  const double ks[3] = {filt ? S.fa : S.aa, filt ? S.fb : S.ab, filt ? S.fc : S.ac};
-  double E[3][7];
-  end_weights(S, filt, E);
-  // amplification, on lines of 56 points (two segments) of both kinds: of every value, of the forward values rows 4..L-4 take in, of values away from
-  // the ends (segment carries), of all values but those of the two end points
-  double amp = 0, amp_u = 0, amp_i = 0, amp_1 = 0;
-  const int L0 = 56;
-  for (int per = 0; per <= (filt ? 0 : 1); per++) {
-    std::vector<double> fc((size_t)L0 * 5);
-    const auto &al = filt ? h->sh.albef : h->sh.albed;
-    penta_factors(al[per], al[per], filt ? h->sh.alphf : 0.5862704032801503, filt ? h->sh.betf : 0.09549533555017055, L0,
-                  fc.data());
-    std::vector<std::vector<double>> R(L0, std::vector<double>(L0, 0.0)), U = R, P = R, D = R, Q = R;
-    for (int i = 0; i < L0; i++) {
-      auto &r = R[i];
-      const int e = i < 3 ? i : (i > L0 - 4 ? L0 - 1 - i : -1);
-      const double sg = !filt && i > 2 ? -1.0 : 1.0;  // a derivative changes sign under reflection
-      auto at = [&](int q) -> double & { return r[i < 3 ? q : L0 - 1 - q]; };
-      if (e < 0) {
-        for (int d = 1; d <= 3; d++) {
-          r[i + d] += ks[d - 1];
-          r[i - d] += filt ? ks[d - 1] : -ks[d - 1];
-          if (filt) r[i] -= 2 * ks[d - 1];
-        }
-      } else if (per && e < 2) {
-        for (int q = 0; q <= LMD; q++) {
-          at(q) += sg * S.pbci[0][e][q];
-          at(L0 - 2 - q) += sg * S.pbco[0][e][q];
-        }
-      } else if (per) {
-        at(3) += sg * ks[0]; at(1) -= sg * ks[0]; at(4) += sg * ks[1]; at(0) -= sg * ks[1];
-        at(5) += sg * ks[2]; at(L0 - 2) -= sg * ks[2];
-      } else {
-        for (int q = 0; q < 7; q++) at(q) += sg * E[e][q];
-      }
-      for (double &v : r) v *= fc[i * 5 + 2];
-    }
-    const int cut = seg_start(1, L0, seg_count(L0));
-    for (int i = 0; i < L0; i++) {
-      const double c2 = fc[i * 5 + 2], l0 = i >= 2 ? c2 * fc[i * 5] / fc[(i - 2) * 5 + 2] : 0;
-      const double l1 = i >= 1 ? c2 * fc[i * 5 + 1] / fc[(i - 1) * 5 + 2] : 0;
-      const int b = i >= cut ? cut : 0;
-      for (int j = 0; j < L0; j++) {
-        U[i][j] = R[i][j] - (i >= 2 ? l0 * U[i - 2][j] : 0) - (i >= 1 ? l1 * U[i - 1][j] : 0);
-        P[i][j] = R[i][j] - (i - 2 >= b ? l0 * P[i - 2][j] : 0) - (i - 1 >= b ? l1 * P[i - 1][j] : 0);
-      }
-    }
-    for (int i = L0 - 1; i >= 0; i--) {
-      const int b = i < cut ? cut : L0;
-      const double c3 = fc[i * 5 + 3], c4 = fc[i * 5 + 4];
-      for (int j = 0; j < L0; j++) {
-        D[i][j] = U[i][j] - (i + 1 < L0 ? c3 * D[i + 1][j] : 0) - (i + 2 < L0 ? c4 * D[i + 2][j] : 0);
-        Q[i][j] = U[i][j] - (i + 1 < b ? c3 * Q[i + 1][j] : 0) - (i + 2 < b ? c4 * Q[i + 2][j] : 0);
-      }
-    }
-    for (int i = 0; i < L0; i++) {
-      for (const auto *M : {&U[i], &P[i]}) {
-        const double v = amplitude(*M, per != 0);
-        amp = std::max(amp, v);
-        if (i >= 2 && i <= L0 - 5) amp_u = std::max(amp_u, v);
-      }
-      for (const auto *M : {&D[i], &Q[i]}) amp = std::max(amp, amplitude(*M, per != 0));
-      for (const auto *M : {&U[i], &P[i], &D[i], &Q[i]}) {
-        const double v = amplitude(*M, per != 0);
-        if (i >= 16 && i < L0 - 16) amp_i = std::max(amp_i, v);
-        if (i >= 1 && i < L0 - 1) amp_1 = std::max(amp_1, v);
-      }
-    }
-  }
-  amp *= 1.0625;  // (other line lengths, rounding)
-  amp_u *= 1.0625;
-  amp_i *= 1.0625;
-  amp_1 *= 1.0625;
-  // the extra scale: a small operator (the filter) uses the range a derivative would
-  T.k = 0;
-  while (T.k < 8 && amp * (2 << T.k) <= 14.0) T.k++;
-  const double sc = (double)(1 << T.k);
-  const double vu = amp_u * sc, vd = amp * sc, vi = amp_i * sc, v1 = amp_1 * sc;  // largest values, in units of the largest difference
-  // the row and end tables of one line; false if a sum of products could leave its range
-  std::vector<double> R, W, G, H;
-  auto line = [&](int L, bool per, const double *fc, int gbits, int *o, int *e, double limit = 9.2e18) {
-    const double g32 = std::ldexp(1.0, gbits - 32);
-    bool fits = true;
-    // a coefficient of a value of up to x differences; mid: the group's largest middle sum so far
-    auto pairc = [&](double c, int *p, double x, double &mid, int bits = FX_BITS) {
-      if (!(std::ldexp(std::fabs(c), bits) < 2147483000.0)) return false;
-      const double hi = std::nearbyint(std::ldexp(c, bits));
-      const double lo = std::min(std::nearbyint(std::ldexp(std::ldexp(c, bits) - hi, 32)), 2147483647.0);
-      p[0] = (int)hi;
-      p[1] = (int)lo;
-      mid += std::fabs(hi) * 2147483648.0 + std::fabs(lo) * (x * g32 + 1.0);
-      return mid < limit;
-    };
-    auto c2 = [&](int i) { return fc[i * 5 + 2]; };
-    auto m0 = [&](int i) { return i >= 2 ? -c2(i) * fc[i * 5] / c2(i - 2) : 0.0; };
-    auto m1 = [&](int i) { return i >= 1 ? -c2(i) * fc[i * 5 + 1] / c2(i - 1) : 0.0; };
-    auto n1 = [&](int i) { return i <= L - 2 ? -fc[i * 5 + 3] : 0.0; };
-    auto n2 = [&](int i) { return i <= L - 3 ? -fc[i * 5 + 4] : 0.0; };
-    for (int i = 0; i < L; i++) {
-      int *r = o + (size_t)i * FX_RT;
-      double f = 0, b = 0;
-      if ((i >= 4 && i <= L - 4) || per) {
-        for (int q = 0; q < 3; q++) fits = fits && pairc(c2(i) * ks[q] * sc, r + 2 * q, 2.0 * (q + 1), f);
-        if (i >= 4 && i <= L - 4) fits = fits && pairc(m0(i), r + 6, vu, f) && pairc(m1(i), r + 8, vu, f);
-      }
-      if (i >= 3) fits = fits && pairc(n1(i), r + 12, vd, b) && pairc(n2(i), r + 14, vd, b);
-    }
-    const int nseg = seg_count(L);
-    for (int k = 0; k < nseg; k++) {  // segment responses (as in seg_tables)
-      const int s0 = seg_start(k, L, nseg), s1 = seg_start(k + 1, L, nseg), n = s1 - s0;
-      for (auto *V : {&R, &W, &G, &H}) V->assign(n + 2, 0.0);
-      if (k > 0) {
-        double g2 = 1, g1 = 0, h2 = 0, h1 = 1;
-        for (int i = s0; i < s1; i++) {
-          R[i - s0] = m0(i) * g2 + m1(i) * g1;
-          W[i - s0] = m0(i) * h2 + m1(i) * h1;
-          g2 = g1; g1 = R[i - s0]; h2 = h1; h1 = W[i - s0];
-          int *r = o + (size_t)i * FX_RT;
-          double mid = 0;
-          fits = fits && pairc(g1, r + 24, vi, mid) && pairc(h1, r + 26, vi, mid);
-        }
-      }
-      if (k < nseg - 1) G[n] = H[n + 1] = 1.0;
-      for (int i = s1 - 1; i >= s0; i--) {
-        const int q = i - s0, cb = filt ? FX_CBITS_FILTER : FX_BITS;
-        for (auto *V : {&R, &W, &G, &H}) (*V)[q] += n1(i) * (*V)[q + 1] + n2(i) * (*V)[q + 2];
-        int *r = o + (size_t)i * FX_RT;
-        double mid = 0;
-        fits = fits && pairc(R[q], r + 16, vi, mid, cb) && pairc(W[q], r + 18, vi, mid, cb) &&
-               pairc(G[q], r + 20, vi, mid, cb) && pairc(H[q], r + 22, vi, mid, cb);
-      }
-    }
-    const double sg = filt ? 1.0 : -1.0;
-    auto endc = [&](double c, int at, double x, double &mid) { return pairc(c, e + 2 * at, x, mid, FX_END_BITS); };
-    for (int r = 0; r < 3; r++) {
-      double ms = 0, me = 0, f = 0, g = 0, b = 0;
-      for (int q = 0, n = 0; q < 7; q++) {
-        if (q == r) continue;
-        const double x = std::abs(q - r);
-        fits = fits && endc(c2(r) * E[r][q] * sc, 6 * r + n, x, ms) &&
-               endc(sg * c2(L - 1 - r) * E[r][q] * sc, 18 + 6 * r + n, x, me);
-        n++;
-      }
-      fits = fits && endc(m0(r), 36 + 2 * r, vd, f) && endc(m1(r), 37 + 2 * r, r == 1 ? vd : v1, f);
-      fits = fits && endc(m0(L - 1 - r), 42 + 2 * r, v1, g) && endc(m1(L - 1 - r), 43 + 2 * r, v1, g);
-      fits = fits && endc(n1(r), 48 + 2 * r, v1, b) && endc(n2(r), 49 + 2 * r, v1, b);
-    }
-    // row 3: next to one-sided rows its c2 is large
-    double m3 = 0, f3 = 0;
-    for (int q = 0; q < 3; q++) fits = fits && endc(c2(3) * ks[q] * sc, 150 + q, 2.0 * (q + 1), m3);
-    fits = fits && endc(m0(3), 153, v1, f3) && endc(m1(3), 154, v1, f3);
-    for (int side = 0; side < 2 && per; side++)
-      for (int r = 0; r < 2; r++) {
-        // weights on f(q) - f(0) and f(L-2-q) - f(0) as weights on the neighbour differences
-        double w[24] = {0};
-        const double c = side ? -c2(L - 1 - r) : c2(r);
-        for (int q = 0; q <= LMD; q++) {
-          for (int j = 0; j < q; j++) w[j] += c * S.pbci[0][r][q] * sc;
-          w[11] += c * S.pbco[0][r][q] * sc;
-          for (int j = 0; j <= q; j++) w[12 + j] += c * S.pbco[0][r][q] * sc;
-        }
-        double mid = 0;
-        for (int q = 0; q < 24; q++) {
-          if (q % 4 == 0) mid = 0;  // (summed four at a time)
-          fits = fits && pairc(w[q], e + 2 * (54 + 48 * side + 24 * r + q), 1.0, mid);
-        }
-      }
-    return fits;
-  };
-  // gbits: the largest for which results stay below 2^63 and every sum in its range, on lines of 13 to 193 points of both
-  // kinds (longer ones repeat these rows; the limit leaves room for segments cut elsewhere): the same for every handle of one scheme, so that a case's results do not
-  // depend on the other cases of a batch
-  std::vector<int> ro, eo(2 * FX_ET);
-  std::vector<double> fct;
-  auto all_fit = [&](int gbits) {
-    if (!(std::ldexp(vd, gbits) < std::ldexp(0.93, 63))) return false;
-    for (int per = 0; per <= (filt ? 0 : 1); per++)
-      for (int L : {13, 14, 25, 48, 49, 72, 97, 120, 152, 193}) {
-        const auto &al = filt ? h->sh.albef : h->sh.albed;
-        fct.resize((size_t)L * 5);
-        penta_factors(al[per], al[per], filt ? h->sh.alphf : 0.5862704032801503, filt ? h->sh.betf : 0.09549533555017055, L,
-                      fct.data());
-        ro.resize((size_t)L * FX_RT);
-        if (!line(L, per != 0, fct.data(), gbits, ro.data(), eo.data(), 8.9e18)) return false;
-      }
-    return true;
-  };
-  T.gbits = 59;
-  while (T.gbits >= 55 && !all_fit(T.gbits)) T.gbits--;
-  T.rows.assign((size_t)(h->nfac + 2 * FX_PAD) * FX_RT, 0);
-  T.ends.assign((size_t)h->nb * 3 * FX_ET, 0);
-  for (int nn = 1; nn <= 3 && T.gbits >= 55; nn++) {  // (below: an extreme filter, the FP64 sweeps take it)
+  if (!h->fix_op[0].gbits) return;
+  for (int nn = 1; nn <= 3; nn++) {
     bool ok = true;
-    for (int gb = 0; gb < h->nb && ok; gb++) {
+    for (int gb = 0; gb < h->nb; gb++) {
       const BlockDev &B = h->blk[gb];
       const int L = nn == 1 ? B.lxi + 1 : (nn == 2 ? B.let + 1 : B.lze + 1);
-      if (!fx_line(L)) continue;  // (this block's lines take the FP64 sweeps)
+      if (!fx_line(L)) continue;
       auto self = [&](int ip) { return B.ndf[ip][nn] == 1 && B.nbc[ip][nn] == 45 && B.ncd[ip][nn] == gb; };
-      const bool per = self(0) && self(1), open = B.ndf[0][nn] == 0 && B.ndf[1][nn] == 0;
-      ok = (open || (per && !filt && nn == 3 && L >= LMD + 2)) &&
-           line(L, per, &fac[(size_t)B.fac_off[nn] * 5], T.gbits, &T.rows[(size_t)(B.fac_off[nn] + FX_PAD) * FX_RT],
-                reinterpret_cast<int *>(&T.ends[((size_t)gb * 3 + nn - 1) * FX_ET]));
+      const bool open = B.ndf[0][nn] == 0 && B.ndf[1][nn] == 0, per = nn == 3 && self(0) && self(1);
+      auto line = [&](int q) {
+        return fix_line(h->sh, h->fix_op[q], q == 1, L, per, &(q ? facf : facd)[(size_t)B.fac_off[nn] * 5],
+                        &h->fix_rows[q][(size_t)(B.fac_off[nn] + FX_PAD) * FX_RT],
+                        reinterpret_cast<int *>(&h->fix_ends[q][((size_t)gb * 3 + nn - 1) * FX_ET]));
+      };
+      // (zeta lines are filtered by the FP64 sweep; an extreme filter takes it in every direction)
+      h->fix_blk[nn][gb] = (open || (per && L >= LMD + 2)) && line(0) && (nn == 3 || !h->fix_op[1].gbits || line(1));
+      ok = ok && h->fix_blk[nn][gb];
     }
-    T.ok[nn] = ok;
+    if (!ok) h->fix_blk[nn].assign(h->nb, 0);
   }
 }
 
@@ -1298,14 +1061,12 @@ static int create_impl(const ati_config_t *cfgs, int ncase, ati_handle_t **out) 
                o_lt2 = take(sizeof(LTile) * h->max_lt[2]), o_lt3 = take(sizeof(LTile) * h->max_lt[3]),
                o_facud = take((size_t)h->nfac * FU_RT * D8), o_facuf = take((size_t)h->nfac * FU_RT * D8);
   // fixed-point line sweeps of the FP64 fast path
-  FixTables fix[2];
   size_t o_fxr[2] = {0, 0}, o_fxe[2] = {0, 0}, o_lts[4] = {0, 0, 0, 0};
   for (int nn = 1; nn <= 3; nn++) o_lts[nn] = take(sizeof(LTile) * std::max<size_t>(h->hlts[nn].size(), 1));
   if (h->cfg.precision == ATI_FP64)
     for (int q = 0; q < 2; q++) {
-      fix_tables(h, q == 1, q ? facf : facd, fix[q]);
-      o_fxr[q] = take(sizeof(int) * fix[q].rows.size());
-      o_fxe[q] = take(sizeof(int64_t) * fix[q].ends.size());
+      o_fxr[q] = take(sizeof(int) * h->fix_rows[q].size());
+      o_fxe[q] = take(sizeof(int64_t) * h->fix_ends[q].size());
     }
   // FP32 set (mixed): de(5) prim(4) mu p(1) dv(12) tau(9) flx(15) fw(3 x 5) xim etm zem(3) yaco asz bsz(1) gm(3)
   size_t o_ff = 0, o_fdrva = 0, o_fdrvb = 0, o_frecv = 0, o_fcm = 0, o_ffacd = 0, o_ffacf = 0, o_fsbcc = 0,
@@ -1367,11 +1128,10 @@ static int create_impl(const ati_config_t *cfgs, int ncase, ati_handle_t **out) 
   d.eta_rowtiles = h->tma[2];
   d.fx_flux = h->cfg.precision != ATI_FP64 || h->cfg.les == 1 ? 0 : (h->cfg.nviscous == 1 ? 1 : 2);
   for (int q = 0; q < 2; q++) {
-    for (int nn = 1; nn <= 3; nn++) d.fx_ok[q][nn] = fix[q].ok[nn];
+    for (int nn = 1; nn <= 3; nn++) d.fx_ok[q][nn] = d.nlt_fx[nn] > 0 && (q == 0 || (nn < 3 && h->fix_op[1].gbits));
     d.fxr[q] = (const int *)(h->arena + o_fxr[q]) + FX_PAD * FX_RT;
     d.fxe[q] = (const int64_t *)(h->arena + o_fxe[q]);
-    d.fx_gbits[q] = fix[q].gbits;
-    d.fx_k[q] = fix[q].k;
+    d.fx_scale[q] = h->fix_op[q];
   }
   h->area = D(o_area); h->wnor = D(o_wnor); h->dforce = D(o_frc); h->dspg = D(o_spg);
   h->dtasks = (FaceTask *)(h->arena + o_task);
@@ -1498,8 +1258,8 @@ static int create_impl(const ati_config_t *cfgs, int ncase, ati_handle_t **out) 
   for (int nn = 1; nn <= 3; nn++) up(d.lts[nn], h->hlts[nn].data(), sizeof(LTile) * h->hlts[nn].size());
   if (h->cfg.precision == ATI_FP64) {
     for (int q = 0; q < 2; q++) {
-      up(d.fxr[q] - FX_PAD * FX_RT, fix[q].rows.data(), sizeof(int) * fix[q].rows.size());
-      up(d.fxe[q], fix[q].ends.data(), sizeof(int64_t) * fix[q].ends.size());
+      up(d.fxr[q] - FX_PAD * FX_RT, h->fix_rows[q].data(), sizeof(int) * h->fix_rows[q].size());
+      up(d.fxe[q], h->fix_ends[q].data(), sizeof(int64_t) * h->fix_ends[q].size());
     }
     if (e == cudaSuccess) e = fast::fixed_init();
   }

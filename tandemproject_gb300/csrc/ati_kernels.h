@@ -7,7 +7,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "ati_fixed_tab.h"
 #include "ati_internal.h"
+#include "ati_seg.h"
 #include "ati_tma.h"
 
 namespace ati {
@@ -64,7 +66,7 @@ struct Eng {
   int nlt_fx[4];        // leading tiles of lt[nn] whose blocks those sweeps take (the others' lines are too short or long)
   const int *fxr[2];
   const int64_t *fxe[2];
-  int fx_gbits[2], fx_k[2];
+  FixScale fx_scale[2];
   int fx_flux;          // its fluxes: 1 viscous, 2 inviscid in fixed point (ati_fixed_flux.h), 0 FP64 (LES; strict mode)
   int sg_lines[4];      // lines per CTA of the eta (2) and zeta (3) sweeps: the tiles of lt[2], lt[3]
   int maxlen[4];        // longest line per direction
@@ -151,15 +153,11 @@ constexpr size_t SG_SMEM_FW = 48 * 1024;
 
 // Segmented line solves of the mixed path: SEG_LINES lines per CTA staged
 // whole in shared memory, each line cut into seg_count(L) segments of about
-// SEG_ROWS points (one warp per segment).  The segmentation is a function of
-// the line length alone, so a block's results do not depend on the other
-// blocks or cases of a handle.  Lines up to SEG_LMAX points fit the tile.
+// SEG_ROWS points (one warp per segment; ati_seg.h).  Lines up to SEG_LMAX
+// points fit the tile.
 constexpr int SEG_LINES = 32, SEG_ROWS = 48, SEG_MAX = 16, SEG_LMAX = 1600;
+static_assert(SEG_ROWS == SEG_CUT && SEG_MAX == SEG_CUTS, "the cut of a line");
 constexpr size_t SEG_SMEM_MAX = 227 * 1024 - 64;  // (a few bytes of static shared memory per kernel)
-__host__ __device__ inline int seg_count(int L) {
-  const int s = (L + SEG_ROWS - 1) / SEG_ROWS;
-  return s < 1 ? 1 : (s > SEG_MAX ? SEG_MAX : s);
-}
 // Row table of the segmented sweeps, SEG_RT floats per LU-factor row:
 //   [0] l0, [1] l1   forward-elimination factors (zero where the row has none)
 //   [4] g, [5] h     the row's forward values from incoming v(s0-2) = 1, v(s0-1) = 1
@@ -181,11 +179,6 @@ constexpr int SEG_PAD = 8;
 //   [8] D = 2 (A + B + C) (the filter's centre weight: its right-hand side is
 //       A (a(i-1) + a(i+1)) + B (a(i-2) + a(i+2)) + C (a(i-3) + a(i+3)) - D a(i)), [9] unused
 constexpr int FU_RT = 10;
-// first row of segment k of S on a line of L points (the first L % S segments hold one row more)
-__host__ __device__ inline int seg_start(int k, int L, int S) {
-  const int q = L / S, r = L % S;
-  return k * q + (k < r ? k : r);
-}
 // Lines of one segment leave a CTA of one warp; SEG_GROUPS groups of SEG_LINES lines then share a CTA (one
 // warp and one tile each), when every line of a direction is one segment long
 constexpr int SEG_GROUPS = 2;
