@@ -930,7 +930,8 @@ static void fu_tables(const ati_handle *h, const std::vector<double> &fac, doubl
 }
 
 // The fixed-point line sweeps (ati_fixed.h) of an FP64 handle: their tables, and the blocks whose lines they take in each
-// direction.
+// direction.  A block is theirs by its own lines alone (their length, ends and coefficients), whatever other blocks or
+// cases the handle holds.
 static void fix_tables(ati_handle *h, const std::vector<double> &facd, const std::vector<double> &facf) {
   for (int nn = 1; nn <= 3; nn++) h->fix_blk[nn].assign(h->nb, 0);
   if (h->cfg.precision != ATI_FP64) return;
@@ -940,8 +941,7 @@ static void fix_tables(ati_handle *h, const std::vector<double> &facd, const std
     h->fix_ends[q].assign((size_t)h->nb * 3 * FX_ET, 0);
   }
   if (!h->fix_op[0].gbits) return;
-  for (int nn = 1; nn <= 3; nn++) {
-    bool ok = true;
+  for (int nn = 1; nn <= 3; nn++)
     for (int gb = 0; gb < h->nb; gb++) {
       const BlockDev &B = h->blk[gb];
       const int L = nn == 1 ? B.lxi + 1 : (nn == 2 ? B.let + 1 : B.lze + 1);
@@ -955,10 +955,7 @@ static void fix_tables(ati_handle *h, const std::vector<double> &facd, const std
       };
       // (zeta lines are filtered by the FP64 sweep; an extreme filter takes it in every direction)
       h->fix_blk[nn][gb] = (open || (per && L >= LMD + 2)) && line(0) && (nn == 3 || !h->fix_op[1].gbits || line(1));
-      ok = ok && h->fix_blk[nn][gb];
     }
-    if (!ok) h->fix_blk[nn].assign(h->nb, 0);
-  }
 }
 
 template <typename T>
