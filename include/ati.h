@@ -343,11 +343,11 @@ int ati_set_tile_plan(ati_handle_t *h, const int32_t plan[ATI_TILE_PLAN]);
  *    one dense L x L product per line, the operator of each block built once
  *    from the line algorithm in FP64, where every zeta face is periodic onto
  *    its own block and lines have 13 to 64 points (else it has no effect).
- *  ATI_OPT_STRESS_AT_POINT: the ATI_FP64 path's viscous fluxes take the
- *    stresses at the point inside the flux kernel instead of writing and
- *    reading nine stress planes (no effect in the strict mode, the mixed path
- *    or with the LES term; the stress output and the forces rebuild the planes
- *    on demand).
+ *  ATI_OPT_STRESS_AT_POINT: kept for callers that set it and reported as set;
+ *    it changes nothing.  The viscous fluxes of the ATI_FP64 path and of the
+ *    mixed path always take the stresses at the point inside the flux kernel
+ *    (the stress output and the forces rebuild the nine stress planes on
+ *    demand); the strict mode and the LES term write and read the planes.
  * *active (may be NULL) gets the options in effect, plus ATI_OPT_TMA_ETA and
  * ATI_OPT_TMA_ZETA for the directions staged by TMA.  Waits for the steps in
  * flight; the step graphs are captured again. */

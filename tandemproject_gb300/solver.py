@@ -307,8 +307,8 @@ class Case:
     def set_options(self, tma=True, fused_faces=False, paired_lines=True, stress_at_point=True, dense_zeta=False):
         """Kernel options (the library's defaults; results do not depend on them, except dense_zeta's by FP32
         rounding): TMA staging of the mixed path's segmented eta/zeta sweeps (a new handle: eta only), fused face
-        chains, paired-line TMA-staged derivative sweeps, the FP64 path's viscous fluxes with the stresses at the
-        point, the mixed path's zeta derivatives as dense products.  Returns the options in effect as a dict."""
+        chains, paired-line TMA-staged derivative sweeps, the mixed path's zeta derivatives as dense products
+        (stress_at_point is reported as set and changes nothing).  Returns the options in effect as a dict."""
         a = ctypes.c_int32()
         flags = ((OPT_TMA if tma else 0) | (OPT_FUSED_FACES if fused_faces else 0)
                  | (OPT_PAIRED_LINES if paired_lines else 0) | (OPT_STRESS_AT_POINT if stress_at_point else 0)
