@@ -2005,12 +2005,11 @@ static int autotune_t(ati_handle *h, Eng<R> &e) {
   // (the mixed path solves every line in segmented tiles of fixed shape: only its point tiles are timed)
   const std::vector<int> sgc{SG_MIN, 2 * SG_MIN, SG_DEFAULT, SG_MAX};
   int sg2 = SG_DEFAULT, sg3 = SG_DEFAULT;
-  // (nor have the fixed-point sweeps of the FP64 fast path tiles to time; the zeta filter keeps the default)
-  const bool fx = !strict && h->ed.fx_ok[0][2] && h->ed.fx_ok[0][3];
-  if (!h->mixed && !fx) {
-    sg2 = pick(sgc, SG_DEFAULT, [&](int v) { set_tiles(v, SG_DEFAULT, PT_DEFAULT); }, sweep_of(2));
-    sg3 = pick(sgc, SG_DEFAULT, [&](int v) { set_tiles(sg2, v, PT_DEFAULT); }, sweep_of(3));
-  }
+  // (nor have the fixed-point sweeps of the FP64 fast path tiles to time, where they take every line of a direction; the
+  // zeta filter, which they leave to the FP64 sweep, then keeps the default: 32 to 256 lines a CTA made no difference to it)
+  auto timed = [&](int nn) { return !h->mixed && (strict || !h->ed.fx_ok[0][nn] || h->ed.nlt_fx[nn] < h->ed.nlt[nn]); };
+  if (timed(2)) sg2 = pick(sgc, SG_DEFAULT, [&](int v) { set_tiles(v, SG_DEFAULT, PT_DEFAULT); }, sweep_of(2));
+  if (timed(3)) sg3 = pick(sgc, SG_DEFAULT, [&](int v) { set_tiles(sg2, v, PT_DEFAULT); }, sweep_of(3));
   set_tiles(sg2, sg3, PT_DEFAULT);
   // point tiles, per pointwise kernel: their best sizes differ (the tile's set-up is a chain of dependent loads
   // that small tiles repeat for every point; large tiles leave a partial last wave of CTAs)

@@ -19,3 +19,23 @@ def test_stress_option_adds_no_launches(ati_lib):
         launches[on] = h.launch_count() - before
     h.close()
     assert launches[True] == launches[False] > 0, launches
+
+
+def test_eta_tiles_are_timed_where_fp64_sweeps_remain(ati_lib):
+    """Lines of under 13 and over 800 points stay with the FP64 eta sweeps, whose lines a CTA ati_init times on the handle's
+    own grid: lines of 851 or 901 points leave shared memory at the default of 128, and fewer lines a CTA are faster by
+    more than the 3 % that a candidate has to be."""
+    from tandemproject_gb300.config import FP64, CaseConfig
+    from tandemproject_gb300.solver import Case
+    import numpy as np
+    from tandemproject_gb300.grid import aerofoil_grid
+    eta = []
+    for lxibk, letbk, lzebk in (((24, 64, 24), (850, 850), (40,)), ((60, 120, 60), (10, 900), (12,))):
+        cfg = CaseConfig(lxibk=lxibk, letbk=letbk, lzebk=lzebk, precision=FP64)
+        h = Case(cfg)
+        for mb, xyz in enumerate(aerofoil_grid(cfg)):
+            h.set_grid(mb, np.ascontiguousarray(xyz))
+        h.init()
+        eta.append(h.tiles()[1])
+        h.close()
+    assert any(n != 128 for n in eta), eta
