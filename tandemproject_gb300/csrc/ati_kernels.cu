@@ -1769,37 +1769,24 @@ __global__ void k_mpigo(const BlockDev *blk, const Coef<TC> *cf, const FaceTask 
 // KEEP: planes that later kernels read again; the others are marked for early eviction.
 template <bool KEEP, typename T>
 __device__ __forceinline__ T ld_stream(const T *p) { return KEEP ? __ldg(p) : __ldcs(p); }
-// V consecutive values at p (V x their size aligned)
+// V = 1 or 2 consecutive values at p (V x their size aligned)
 template <int V, bool KEEP = false>
 __device__ __forceinline__ void vload(float (&o)[V], const float *p) {
+  static_assert(V <= 2, "single points or pairs");
   if constexpr (V == 1) o[0] = ld_stream<KEEP>(p);
-  else if constexpr (V == 2) { const float2 v = ld_stream<KEEP>(reinterpret_cast<const float2 *>(p)); o[0] = v.x; o[1] = v.y; }
-  else { const float4 v = ld_stream<KEEP>(reinterpret_cast<const float4 *>(p)); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+  else { const float2 v = ld_stream<KEEP>(reinterpret_cast<const float2 *>(p)); o[0] = v.x; o[1] = v.y; }
 }
 template <int V, bool KEEP = false>
 __device__ __forceinline__ void vload(double (&o)[V], const double *p) {
+  static_assert(V <= 2, "single points or pairs");
   if constexpr (V == 1) o[0] = ld_stream<KEEP>(p);
-  else {
-#pragma unroll
-    for (int k = 0; k < V; k += 2) {
-      const double2 v = ld_stream<KEEP>(reinterpret_cast<const double2 *>(p + k));
-      o[k] = v.x; o[k + 1] = v.y;
-    }
-  }
+  else { const double2 v = ld_stream<KEEP>(reinterpret_cast<const double2 *>(p)); o[0] = v.x; o[1] = v.y; }
 }
-template <int V>
-__device__ __forceinline__ void vstore(double *p, const double (&v)[V]) {
+template <int V, typename T>
+__device__ __forceinline__ void vstore(T *p, const T (&v)[V]) {
+  static_assert(V == 1 || (V == 2 && sizeof(T) == 4), "single points, or pairs of FP32 values");
   if constexpr (V == 1) *p = v[0];
-  else {
-#pragma unroll
-    for (int k = 0; k < V; k += 2) *reinterpret_cast<double2 *>(p + k) = make_double2(v[k], v[k + 1]);
-  }
-}
-template <int V>
-__device__ __forceinline__ void vstore(float *p, const float (&v)[V]) {
-  if constexpr (V == 1) *p = v[0];
-  else if constexpr (V == 2) *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
-  else *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
 }
 
 // the points of tile T in groups of V consecutive ones, the first group from a multiple of V; a group at a tile's end
