@@ -3400,8 +3400,13 @@ static void pointwise_t(const Eng<R> &eng, cudaStream_t st, int which) {
       }
       break;
     case PW_DIV:
-      if (Freestream<R>::on && e.N % 2 == 0) k_div<R, 2><<<g, t, 0, st>>>(e);
-      else k_div<R, 1><<<g, t, 0, st>>>(e);
+      if constexpr (Freestream<R>::on) {
+        if (e.N % 2 == 0) {
+          k_div<R, 2><<<g, t, 0, st>>>(e);
+          break;
+        }
+      }
+      k_div<R, 1><<<g, t, 0, st>>>(e);
       break;
     case PW_RK:
       k_rk<R><<<g, t, 0, st>>>(e);
