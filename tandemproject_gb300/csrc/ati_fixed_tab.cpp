@@ -82,7 +82,8 @@ double amplitude(const std::vector<double> &c, bool per) {
   double best = 0, s = 0;
   for (int j = L - 1; j >= 1; j--) best += std::fabs(s += c[j]);
   if (!per) return best;
-  for (int m = 0; m < L - 1; m++) {  // points up to m reached from point 0, the others from the far end
+  // points up to m reached from point 0, the others from the far end (any m bounds the row; three are tried)
+  for (int m = L / 4; m < L - 1; m += L / 4) {
     double t = 0, v = 0;
     for (int j = m; j >= 1; j--) t += std::fabs(v += c[j]);
     v = 0;
@@ -281,22 +282,29 @@ bool fix_line(const SchemeHost &H, const FixOp &op, bool filt, int L, bool per, 
 
 FixOp fix_operator(const SchemeHost &H, bool filt) {
   // the lines that the bounds and the sums are checked on: every cut into groups, one to five segments, both kinds
-  std::vector<int> lens;
-  for (int L = FX_LMIN; L <= 50; L++) lens.push_back(L);
-  for (int L : {56, 63, 72, 97, 120, 152, 193}) lens.push_back(L);
+  struct Line {
+    int L;
+    bool per;
+    std::vector<double> fac;
+  };
+  std::vector<Line> lines;
+  auto line = [&](int L) {
+    for (int per = 0; per <= (filt ? 0 : 1); per++) lines.push_back({L, per != 0, factors_of(H, filt, L, per != 0)});
+  };
+  for (int L = FX_LMIN; L <= 31; L++) line(L);
+  for (int L : {48, 49, 50, 57, 63, 97, 120}) line(L);
   FixBounds B;
-  for (int per = 0; per <= (filt ? 0 : 1); per++)
-    for (int L : lens) {
-      const FixBounds b = fix_bounds(H, filt, L, per != 0);
-      for (int z = 0; z < 2; z++) {
-        const int y = per ? 0 : z;  // (a periodic line's last group is like the others)
-        B.forward[y] = std::max(B.forward[y], b.forward[z]);
-        B.inner[y] = std::max(B.inner[y], b.inner[z]);
-        B.forward_carry[y] = std::max(B.forward_carry[y], b.forward_carry[z]);
-        B.backward[y] = std::max(B.backward[y], b.backward[z]);
-        B.backward_carry[y] = std::max(B.backward_carry[y], b.backward_carry[z]);
-      }
+  for (const Line &l : lines) {
+    const FixBounds b = fix_bounds(H, filt, l.L, l.per);
+    for (int z = 0; z < 2; z++) {
+      const int y = l.per ? 0 : z;  // (a periodic line's last group is like the others)
+      B.forward[y] = std::max(B.forward[y], b.forward[z]);
+      B.inner[y] = std::max(B.inner[y], b.inner[z]);
+      B.forward_carry[y] = std::max(B.forward_carry[y], b.forward_carry[z]);
+      B.backward[y] = std::max(B.backward[y], b.backward[z]);
+      B.backward_carry[y] = std::max(B.backward_carry[y], b.backward_carry[z]);
     }
+  }
   FixOp op;
   // the extra scale: a small operator (the filter) uses the range a derivative would
   while (op.k < 8 && std::max(B.forward[0], B.backward[0]) * (2 << op.k) <= 14.0) op.k++;
@@ -308,13 +316,9 @@ FixOp fix_operator(const SchemeHost &H, bool filt) {
     op.vinner = std::max(B.inner[0] * sc + B.forward_carry[0] * c, B.inner[1] * sc * d + B.forward_carry[1] * ce);
     op.vback = std::max(B.backward[0] * sc + B.backward_carry[0] * c, B.backward[1] * sc * d + B.backward_carry[1] * ce);
     if (!(std::max(op.vfwd, op.vback) < most)) return false;
-    std::vector<int> ro, eo(2 * FX_ET);
-    for (int per = 0; per <= (filt ? 0 : 1); per++)
-      for (int L : lens) {
-        const std::vector<double> fc = factors_of(H, filt, L, per != 0);
-        ro.assign((size_t)L * FX_RT, 0);
-        if (!fix_line(H, op, filt, L, per != 0, fc.data(), ro.data(), eo.data())) return false;
-      }
+    std::vector<int> ro((size_t)lines.back().L * FX_RT), eo(2 * FX_ET);
+    for (const Line &l : lines)
+      if (!fix_line(H, op, filt, l.L, l.per, l.fac.data(), ro.data(), eo.data())) return false;
     return true;
   };
   // The unit's size sets the error, 2^-gbits of the differences that a group reads or 2^-carry of the values carried in,
