@@ -29,17 +29,17 @@ constexpr int FX_PAD = 8;  // rows of zero padding on each side of the table (re
 constexpr int FX_ET = 156;
 constexpr int FX_END_BITS = 24;
 // A segment's rows fall into groups, whose values share one scale: of FX_GR rows, the last one too; what does not divide is
-// a group of its own before the last one (five to seven rows) or goes with the one there (up to twelve).  Values change by
-// a factor of 0.73 a row at most where nothing drives them, 3.6 bits a group, which the integers' spare bits over FP64's
-// cover.  The first and the last group hold the seven points that one-sided end rows read, the two groups at either end
-// the thirteen of a periodic line's.
+// a group of its own before the last one (five to seven rows) or goes with the one there (up to twelve); up to 15 rows are
+// one group.  Values change by a factor of 0.73 a row at most where nothing drives them, 3.6 bits a group, which the
+// integers' spare bits over FP64's cover.  The first and the last group hold the seven points that one-sided end rows read,
+// the two groups at either end the thirteen of a periodic line's.
 constexpr int FX_GR = 8;
 ATI_HD int fx_groups(int n) {
-  return n < 14 ? 1 : (n == 14 ? 2 : (n - FX_GR) / FX_GR + ((n - FX_GR) % FX_GR >= 5) + 1);
+  return n < 2 * FX_GR ? 1 : (n - FX_GR) / FX_GR + ((n - FX_GR) % FX_GR >= 5) + 1;
 }
 // rows before group g of ng in a segment of n rows (g = ng: n)
 ATI_HD int fx_group_start(int g, int ng, int n) {
-  return g < ng - 1 || g == 0 ? FX_GR * g : (g == ng ? n : (n == 14 ? 7 : n - FX_GR));
+  return g < ng - 1 || g == 0 ? FX_GR * g : (g == ng ? n : n - FX_GR);
 }
 // values carried from segment to segment stay below 2^FX_CARRY
 constexpr int FX_CARRY = 59;
