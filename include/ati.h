@@ -408,7 +408,8 @@ int ati_check_recip(int64_t n, double worst[2]);
  * asynchronously on `stream` (a cudaStream_t; NULL = the legacy default
  * stream).
  *  - Allocates and frees nothing.  Its scratch (LU factors; the
- *    forward-elimination values stay in shared memory) is one static device
+ *    forward-elimination values stay in shared memory, short lines' in out) is
+ *    one static device
  *    array of 5*ATI_NOALLOC_MAX_LEN + 1 doubles (160 KB) per GPU, held until the
  *    process exits.
  *  - The first call on each device (and again after a device reset, which

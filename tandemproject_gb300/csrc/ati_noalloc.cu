@@ -8,7 +8,8 @@
 // caller passes its own input and output arrays, and the only extra memory
 // the kernel needs -- the LU factor table -- lives in the file-scope device
 // array below (160 KB on every GPU that uses it, held until the process exits);
-// the forward-elimination values stay in shared memory.  No call allocates or frees anything.
+// the forward-elimination values stay in shared memory, those of short lines in
+// the output.  No call allocates or frees anything.
 //
 // When the array is reserved: with CUDA's default lazy module loading this file's
 // module, and the array with it, is loaded into a context the first time the
@@ -182,6 +183,77 @@ __global__ void __launch_bounds__(kThreads) k_noalloc_deriv(const double *in, do
     for (int i = t; i < L; i += kThreads) q0[(int64_t)ln * L + i] = tile[ln * P + i];
 }
 
+// Short lines: one thread a line straight on the caller's arrays, the forward values in out (a row's forward value is
+// stored when its window has been read, so in may be out).  A tile of n lines costs the same for 7 points a line as for
+// some 2 n + 4, its threads idle, and there one thread a line is as fast or faster: measured, us a call, this kernel and
+// the tiles: 40 lines of 7 9.3 and 12.4, 5,000 of 16 17.2 and 24.7 (of 48: 45 and 35), 30,000 of 32 51 and 59, 200,000 of 7
+// 70 and 223.
+constexpr int kLineThreads = 128;
+__global__ void __launch_bounds__(kLineThreads) k_noalloc_line(const double *in, double *out, int64_t nlines, int len,
+                                                               const double *fac, Rows R) {
+  const int64_t t = blockIdx.x * (int64_t)kLineThreads + threadIdx.x;
+  if (t >= nlines) return;
+  const int L = len;
+  const double *p = in + t * L;
+  double *o = out + t * L;
+  // (the same sums from both ends; from the far one the differences are taken the other way round)
+  double sb[2][3];
+#pragma unroll
+  for (int end = 0; end < 2; end++) {
+    double w[7];
+#pragma unroll
+    for (int q = 0; q < 7; q++) w[q] = p[end ? L - 1 - q : q];
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      double v = 0;
+#pragma unroll
+      for (int q = 0, n = 0; q < 7; q++) {
+        if (q == r) continue;
+        const double x = R.abc[r][n] * (end ? w[r] - w[q] : w[q] - w[r]);
+        v = n == 0 ? x : v + x;
+        n++;
+      }
+      sb[end][r] = v;
+    }
+  }
+  double a0 = p[0], a1 = p[1], a2 = p[2], a3 = p[3], a4 = p[4], a5 = p[5];
+  double f2 = sb[0][0], f1 = sb[0][1] - fac[6] * f2;
+  const double g2 = sb[0][2] - fac[10] * f2 - fac[11] * f1;
+  const double p6 = p[6];
+  o[0] = f2;
+  o[1] = f1;
+  o[2] = g2;
+  f2 = f1;
+  f1 = g2;
+  for (int i = 3; i <= L - 4; i++) {
+    const double a6 = i == 3 ? p6 : p[i + 3];
+    const double s = kAa * (a4 - a2) + kAb * (a5 - a1) + kAc * (a6 - a0);
+    const double v = s - fac[i * 5] * f2 - fac[i * 5 + 1] * f1;
+    o[i] = v;
+    f2 = f1;
+    f1 = v;
+    a0 = a1; a1 = a2; a2 = a3; a3 = a4; a4 = a5; a5 = a6;
+  }
+#pragma unroll
+  for (int r = 2; r >= 0; r--) {
+    const int i = L - 1 - r;
+    const double v = sb[1][r] - fac[i * 5] * f2 - fac[i * 5 + 1] * f1;
+    if (r == 2) o[i] = v;
+    f2 = f1;
+    f1 = v;
+  }
+  double b0 = fac[(L - 1) * 5 + 2] * f1;
+  double b1 = fac[(L - 2) * 5 + 2] * f2 - fac[(L - 2) * 5 + 3] * b0;
+  o[L - 1] = b0;
+  o[L - 2] = b1;
+  for (int i = L - 3; i >= 0; i--) {
+    const double v = fac[i * 5 + 2] * o[i] - fac[i * 5 + 3] * b1 - fac[i * 5 + 4] * b0;
+    o[i] = v;
+    b0 = b1;
+    b1 = v;
+  }
+}
+
 // lines a CTA: the fewest (4 to 32) that leave at most one recurrence warp a sub-partition of the device, within the
 // shared memory of a CTA
 constexpr size_t kTileMax = 200 * 1024;
@@ -191,6 +263,9 @@ int lines_per_cta(int64_t nlines, int len, int nsm) {
   while (lpc > 4 && (size_t)lpc * (len | 1) * sizeof(double) > kTileMax) lpc /= 2;
   return lpc;
 }
+
+// short lines take k_noalloc_line (see there)
+bool one_thread_a_line(int len, int lpc) { return len <= 2 * lpc + 4; }
 
 std::mutex g_mu;
 // per device: the scratch array's device address, the context it was looked up in, and the line length whose
@@ -330,7 +405,11 @@ extern "C" int ati_deriv_lines_noalloc(const double *in, double *out, int64_t nl
   if (refactor) k_noalloc_factors<<<1, 1, 0, st>>>(fac, len, R);
   const int lpc = lines_per_cta(nlines, len, nsm);
   const size_t smem = (size_t)lpc * (len | 1) * sizeof(double);
-  k_noalloc_deriv<<<(unsigned)((nlines + lpc - 1) / lpc), kThreads, smem, st>>>(in, out, nlines, len, lpc, nsm, fac, R);
+  if (one_thread_a_line(len, lpc))
+    k_noalloc_line<<<(unsigned)((nlines + kLineThreads - 1) / kLineThreads), kLineThreads, 0, st>>>(in, out, nlines, len,
+                                                                                                    fac, R);
+  else
+    k_noalloc_deriv<<<(unsigned)((nlines + lpc - 1) / lpc), kThreads, smem, st>>>(in, out, nlines, len, lpc, nsm, fac, R);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     std::lock_guard<std::mutex> lk(g_mu);
