@@ -60,14 +60,16 @@ POINTWISE_BYTES_MIXED = {"flux": 208}
 # fields swept per direction per time step: 4 viscous gradients + 5 fluxes in
 # each of the 4 stages, or the 5 variables once for the filter
 FIELD_SWEEPS_PER_STEP = {"deriv": 4 * (4 + 5), "filter": 5}
-# DRAM bytes per unit of the FP64 xi derivative sweep measured with ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum of one 5-field launch on the
-# 3.54 M-point case: 489.35 MB for 17.69 M units); the kernel streams, so the
-# traffic of a launch scales with the units it processes
-SWEEP_TRAFFIC_PER_UNIT = {"deriv_xi": 489.35e6 / (5 * 3538944)}
-# DRAM bytes per point of the viscous flux kernel (k_flux_fixed) measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum of one launch
-# on the 3.54 M-point case: 906.4 + 395.5 MB); the kernel streams, so the traffic scales with the points
-FLUX_TRAFFIC_PER_POINT = (906.36e6 + 395.46e6) / 3538944
+# DRAM bytes per unit of the FP64 derivative sweeps (k_sweep_fix) measured with ncu (dram__bytes_read.sum +
+# dram__bytes_write.sum of one 5-field launch each on a case of 3,563,520 points,
+# profiles/fixed_point_and_pairs_naca0012_3p6m.md; a part of the writes stays in L2); the kernel streams, so the traffic
+# of a launch scales with the units it processes
+NCU_POINTS = 3563520
+SWEEP_TRAFFIC_PER_UNIT = {"deriv_xi": (142.8e6 + 81.8e6) / (5 * NCU_POINTS),
+                          "deriv_eta": (143.0e6 + 85.8e6) / (5 * NCU_POINTS),
+                          "deriv_zeta": (142.7e6 + 90.9e6) / (5 * NCU_POINTS)}
+# DRAM bytes per point of the viscous flux kernel (k_flux_fixed), the same capture
+FLUX_TRAFFIC_PER_POINT = (912.8e6 + 402.9e6) / NCU_POINTS
 # algorithmic bytes per point of the FP64 fast path's viscous flux kernel k_flux_fixed (the stresses of k_visc taken
 # at the point): it reads the metrics (72 B), the twelve derivative planes of u, v, w, T (96 B), Jacobian and
 # viscosity (16 B), velocity (24 B), pressure (8 B) and the state (40 B), and writes 15 fluxes (120 B)
@@ -504,11 +506,11 @@ def main():
         ach64 = SWEEP_FLOPS[kind] * units / t / 1e12
         return {"bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
                 "traffic": SWEEP_TRAFFIC_PER_UNIT[cls] * units if cls in SWEEP_TRAFFIC_PER_UNIT else None,
-                "traffic_source": "ncu DRAM bytes per unit of one launch on the 3.54 M-point case, scaled by units",
+                "traffic_source": "ncu DRAM bytes per unit of one launch on a case of 3.56 M points, scaled by units",
                 "kernel": f"k_sweep<{cls}>: one launch = every line of one direction over all blocks for "
                           f"{units / npts:.1f} fields on average ({units:.3e} point-fields), "
-                          f"{SWEEP_BYTES[kind]} B and {SWEEP_FLOPS[kind]} flop per point-field",
-                "fp64": {"achieved_tflops": ach64, "peak_tflops": fp64_peak, "frac": ach64 / fp64_peak}}
+                          f"{SWEEP_BYTES[kind]} B and the work of {SWEEP_FLOPS[kind]} flop per point-field",
+                "fp64_equivalent": {"tflops": ach64, "fp64_fma_peak_tflops": fp64_peak}}
 
     sweep_cls = max((k for k in prof if k.startswith(("deriv", "filter")) and prof[k][1]), key=lambda k: prof[k][0])
     if dom == "flux" and cfg.nviscous == 1:
@@ -520,21 +522,22 @@ def main():
         roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                     "frac": achieved / hbm_peak,
                     "traffic": FLUX_TRAFFIC_PER_POINT * npts if FLUX_TRAFFIC_PER_POINT else None,
-                    "traffic_source": "ncu DRAM bytes per point of one launch on the 3.54 M-point case, scaled by "
+                    "traffic_source": "ncu DRAM bytes per point of one launch on a case of 3.56 M points, scaled by "
                                       "points",
                     "kernel": f"k_flux_fixed (viscous fluxes with the stresses at the point): one launch = every point "
-                              f"({npts}), {FLUX_BYTES_FP64} B and {FLUX_FLOPS_FP64} FP64 flop per point",
-                    "fp64": {"achieved_tflops": fp64_ach, "peak_tflops": fp64_peak, "frac": fp64_ach / fp64_peak}}
+                              f"({npts}), {FLUX_BYTES_FP64} B and the work of {FLUX_FLOPS_FP64} FP64 flop per point",
+                    "fp64_equivalent": {"tflops": fp64_ach, "fp64_fma_peak_tflops": fp64_peak}}
     elif dom.startswith(("deriv", "filter")):
         roofline = sweep_roofline(dom)
     else:  # (a class with no algorithmic count leads only when launches are serialised, e.g. under a profiler)
         roofline = sweep_roofline(sweep_cls)
         roofline["note"] = f"largest class {dom} has no algorithmic byte count; the largest sweep class is shown"
-    roofline["fp64"]["peak_source"] = "measured FP64 FMA throughput of this GPU (ati_probe_fma_tflops)"
+    roofline["fp64_equivalent"]["peak_source"] = "measured FP64 FMA throughput of this GPU (ati_probe_fma_tflops)"
     roofline.update({
         "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)",
         "limit": "integer issue: the line sweeps and the fluxes run in 64-bit fixed point on the integer pipes; frac is "
-                 "against HBM, fp64 the rate of the same work counted in FP64 operations against the FP64 FMA peak",
+                 "against HBM; fp64_equivalent is the rate of the work counted in the FP64 operations it replaces, which "
+                 "the kernel does not execute, beside the FP64 FMA peak",
         "stage_hbm_frac": STAGE_BYTES_FP64 * value / ws / 1e9 / hbm_peak,
         "kernel_share": {k: round(v[0] / tot, 4) for k, v in prof.items() if v[1]}})
     if dom != sweep_cls and "note" not in roofline:

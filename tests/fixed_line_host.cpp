@@ -2,7 +2,9 @@
 // against extended precision.  Arguments: operator (0 derivative, 1 filter), periodic, points, kind of line, log2 of the
 // kind's scale, number of lines, seed.  Output: the largest and the mean over the line's points of the ratio of the two
 // root mean square errors over the lines, then the ratio over all points and lines, then the largest integer of the solve
-// in bits (63: overflow).
+// in bits (63: overflow).  Or "scales", operator, filter cut-off: the scales (0: left to FP64), and per line length the
+// largest value that a group's rows can reach, in bits.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -167,7 +169,28 @@ static std::vector<double> fixed(const std::vector<double> &f, const std::vector
   return out;
 }
 
+static int scales(bool filt, double fltk) {
+  ati_config_t cfg{};
+  cfg.fltk = cfg.fltkbc = fltk;
+  build_scheme(cfg, H);
+  const FixOp op = fix_operator(H, filt);
+  printf("%d %d %d %d %d\n", op.gbits, op.k, op.carry, op.spare, op.carry_end);
+  for (int L : {13, 15, 16, 22, 49, 97, 241, 800})
+    for (int per = 0; per <= (filt ? 0 : 1) && op.gbits; per++) {
+      const FixBounds b = fix_bounds(H, filt, L, per != 0);
+      double top = 0;
+      for (int z = 0; z < 2; z++) {
+        const bool end = z && !per;  // an open line's last group
+        const double sc = std::ldexp(1.0, op.gbits + op.k - (end ? op.spare : 0)), c = std::ldexp(1.0, end ? op.carry_end : op.carry);
+        top = std::max({top, b.forward[z] * sc + b.forward_carry[z] * c, b.backward[z] * sc + b.backward_carry[z] * c});
+      }
+      printf("%d %d %.4f\n", L, per, std::log2(top));
+    }
+  return 0;
+}
+
 int main(int argc, char **argv) {
+  if (argc == 4 && !std::strcmp(argv[1], "scales")) return scales(atoi(argv[2]) != 0, atof(argv[3]));
   if (argc < 8) return 2;
   const bool filt = atoi(argv[1]) != 0, per = atoi(argv[2]) != 0;
   const int L = atoi(argv[3]), kind = atoi(argv[4]), scale = atoi(argv[5]), n = atoi(argv[6]);

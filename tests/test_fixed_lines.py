@@ -91,3 +91,23 @@ def test_filter_cut_offs(program, fltk):
 def test_extreme_filters_are_left_to_the_fp64_sweeps(program, fltk):
     out = subprocess.run([program, "1", "0", "97", "0", "0", "1", "1", str(fltk)], capture_output=True)
     assert out.returncode == 3
+
+
+@pytest.mark.parametrize("op,fltk", [(0, 0.85), (1, 0.5), (1, 0.6), (1, 0.7), (1, 0.85), (1, 0.9), (1, 0.93)])
+def test_scales_leave_room_at_every_length(program, op, fltk):
+    """The scales an operator gets: 57 to 60 bits for differences, and no value of a group's rows above 2^62.9 on lines of 13
+    to 800 points, open or periodic, by the bound that holds for any line."""
+    out = subprocess.run([program, "scales", str(op), str(fltk)], check=True, capture_output=True, text=True).stdout
+    head, *rows = [line.split() for line in out.splitlines()]
+    gbits, k, carry, spare, carry_end = map(int, head)
+    assert 57 <= gbits <= 60 and 0 <= k <= 8 and 56 <= carry <= 60 and spare <= 2 and carry_end >= 56, head
+    assert len(rows) == 8 * (2 - op)
+    for length, per, bits in rows:
+        assert float(bits) < 62.9, (length, per, bits)
+
+
+@pytest.mark.parametrize("fltk", [0.3, 0.45, 0.95])
+def test_scales_of_filters_that_do_not_fit(program, fltk):
+    """Cut-offs below some 0.5 and above some 0.93 of the grid's limit: no scales, the FP64 sweeps filter."""
+    out = subprocess.run([program, "scales", "1", str(fltk)], check=True, capture_output=True, text=True).stdout
+    assert out.split()[0] == "0"
