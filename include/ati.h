@@ -409,9 +409,8 @@ int ati_check_recip(int64_t n, double worst[2]);
  * stream).
  *  - Allocates and frees nothing.  Its scratch (LU factors; the
  *    forward-elimination values stay in shared memory, short lines' in out) is
- *    one static device
- *    array of 5*ATI_NOALLOC_MAX_LEN + 1 doubles (160 KB) per GPU, held until the
- *    process exits.
+ *    one static device array of 5*ATI_NOALLOC_MAX_LEN + 1 doubles (160 KB) per
+ *    GPU, held until the process exits.
  *  - The first call on each device (and again after a device reset, which
  *    gives the context a new array) looks up the array's device address with
  *    cudaGetSymbolAddress, that device current.  Under CUDA's default lazy

@@ -10,9 +10,10 @@
 // multiply-adds of 4 clocks, at 15 warps an SM (128 registers a thread; the tiles fill the shared memory): half of the
 // issue slots, the FP64 pipe a sixth busy with the conversions out, DRAM at 20-25 %.  Clocks a row of a warp, of some 1700
 // along eta: staging 150, scales and conversions 320, elimination 570, back substitution 320, results 390.  On 8.85 M
-// points (4.5 fields a launch, 2070 MHz): xi 795 -> 497 us, eta 754 -> 487, zeta 764 -> 405 a derivative launch, the xi and
-// eta filters 1093 -> 580 and 954 -> 620, against the FP64 sweeps (k_sweep_xc, k_sweep_g), which keep the FP64 pipe 86-91 % busy.  (With
-// one scale for a whole line: xi 450, eta 384, zeta 385, but rows well below the line's largest lost accuracy.)
+// points (4.5 fields a launch, 2070 MHz): xi 795 -> 500 us, eta 754 -> 486, zeta 764 -> 407 a derivative launch, the xi and
+// eta filters 1093 -> 583 and 954 -> 625, against the FP64 sweeps (k_sweep_xc, k_sweep_g), which keep the FP64 pipe
+// 86-91 % busy.  (With one scale for a whole line: xi 450, eta 384, zeta 385, but rows well below the line's largest lost
+// accuracy.)
 #include <cuda_runtime.h>
 
 #include <cstdint>
